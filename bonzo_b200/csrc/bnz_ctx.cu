@@ -1327,18 +1327,15 @@ bool split_map(const bnz_ctx* c, const double* base, int nft, int bx, int by, in
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// The split kernels' maps into device memory, when every map can be made, in
-// the order of split::TM_*: for the update (boxes of 34 x 9 cells, 1 or 2
-// planes) prim, the three flux arrays, bfld, the b^n copy in ec, ee; for the
-// corrector's PLM flux tiles, the predictor's prim in cons_s in the boxes of
-// the x (34 x 8 x 1), y (16 x 18 x 1) and z (16 x 1 x 18) sweeps.
+// The split update's maps into device memory, when every map can be made, in
+// the order of split::TM_* (boxes of 34 x 9 cells, 1 or 2 planes): prim, the
+// three flux arrays, bfld, the b^n copy in ec, ee.
 cudaError_t build_split_maps(bnz_ctx* c) {
-  CUtensorMap m[10];
+  CUtensorMap m[7];
   const bool ok = split_map(c, c->prim, 9, 34, 9, 1, 9, &m[0]) && split_map(c, c->flx[0], 9, 34, 9, 1, 6, &m[1]) &&
                   split_map(c, c->flx[1], 9, 34, 9, 1, 6, &m[2]) && split_map(c, c->flx[2], 9, 34, 9, 2, 6, &m[3]) &&
                   split_map(c, c->bfld, 3, 34, 9, 2, 3, &m[4]) && split_map(c, c->ec, 3, 34, 9, 2, 3, &m[5]) &&
-                  split_map(c, c->ee, 3, 34, 9, 2, 3, &m[6]) && split_map(c, c->cons_s, 9, 34, 8, 1, 9, &m[7]) &&
-                  split_map(c, c->cons_s, 9, 16, 18, 1, 9, &m[8]) && split_map(c, c->cons_s, 9, 16, 1, 18, 9, &m[9]);
+                  split_map(c, c->ee, 3, 34, 9, 2, 3, &m[6]);
   if (!ok) return cudaSuccess;  // the kernel without TMA runs
   cudaError_t e = cudaMalloc((void**)&c->d_smaps, sizeof m);
   if (e == cudaSuccess) e = cudaMemcpy(c->d_smaps, m, sizeof m, cudaMemcpyHostToDevice);

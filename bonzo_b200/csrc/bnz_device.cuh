@@ -16,6 +16,9 @@
 #ifndef BNZ_NM
 #define BNZ_NM 9
 #endif
+#ifndef BNZ_FAST_MATH
+#define BNZ_FAST_MATH 0
+#endif
 
 namespace dev {
 
@@ -49,9 +52,8 @@ __device__ __forceinline__ void cons2prim(double* w, const double* u, double gam
   w[BZ] = u[BZ];
 }
 
-// eos_c.h:60-95
-__device__ __forceinline__ void prim2cons(double* u, const double* w, double gam) {
-  double gamm1i = 1. / (gam - 1.);
+// eos_c.h:60-95; gamm1i = 1 / (gam - 1)
+__device__ __forceinline__ void prim2cons_g(double* u, const double* w, double gamm1i) {
   u[RHO] = w[RHO];
   u[MX] = w[RHO] * w[VX];
   u[MY] = w[RHO] * w[VY];
@@ -63,6 +65,10 @@ __device__ __forceinline__ void prim2cons(double* u, const double* w, double gam
   u[BX] = w[BX];
   u[BY] = w[BY];
   u[BZ] = w[BZ];
+}
+
+__device__ __forceinline__ void prim2cons(double* u, const double* w, double gam) {
+  prim2cons_g(u, w, 1. / (gam - 1.));
 }
 
 // eos_c.h:416-461 with a = 1 (no pressure anisotropy)
@@ -107,9 +113,10 @@ __device__ __forceinline__ double rcp_nr(double x) {
 }
 
 #if BNZ_FAST_MATH
-// fms of both face states with one division for the two 0.5 / rho
+// the larger fms of both face states, with one division for the two 0.5 / rho
+// and one square root, of the larger square (the root is monotonic)
 template <bool NR = false>
-__device__ __forceinline__ void fms2(const double* wL, const double* wR, double gam, double& cfL, double& cfR) {
+__device__ __forceinline__ double fms2(const double* wL, const double* wR, double gam) {
   const double h = NR ? 0.5 * rcp_nr<NR>(wL[RHO] * wR[RHO]) : 0.5 / (wL[RHO] * wR[RHO]);
   double q[2];
 #pragma unroll
@@ -122,8 +129,7 @@ __device__ __forceinline__ void fms2(const double* wL, const double* wR, double 
     double c2 = sqrt(fabs(c1 * c1 - 4. * gamp * bx2));
     q[s] = (s ? wL[RHO] : wR[RHO]) * h * (c1 + c2);
   }
-  cfL = sqrt(q[0]);
-  cfR = sqrt(q[1]);
+  return sqrt(fmax(q[0], q[1]));
 }
 #endif
 
@@ -132,13 +138,12 @@ template <bool NR = false>
 __device__ __forceinline__ void wave_speeds(const double* wL, const double* wR, double gam,
                                             double& sL, double& sR) {
 #if BNZ_FAST_MATH
-  double cfL, cfR;
-  fms2<NR>(wL, wR, gam, cfL, cfR);
+  double cf_max = fms2<NR>(wL, wR, gam);
 #else
   double cfL = fms(wL, gam);
   double cfR = fms(wR, gam);
-#endif
   double cf_max = fmax(cfL, cfR);
+#endif
   sL = fmin(wL[VX], wR[VX]) - cf_max;
   sR = fmax(wL[VX], wR[VX]) + cf_max;
 }
@@ -348,10 +353,19 @@ __device__ __forceinline__ void flux_hllt(double* flux, const double* wL, const 
 // 9-vectors are evaluated once -- about half the live registers of forming
 // both sides, with no warp divergence.  NR (fast build only): the five
 // reciprocals by bnz_nr_rcp instead of IEEE divisions.
-template <bool NR = false>
-__device__ __forceinline__ void flux_hlld(double* flux, const double* wL, const double* wR, double gam,
-                                          unsigned& err) {
-  const double bx = wL[BX];
+// St gives the face states: L(n), R(n), and at(left, n) of the side picked,
+// which the kernels that keep the states in shared memory read there again
+// (an address picked per lane instead of a select per value).  bx: the normal
+// field of both (n = BX is not asked of St).  gm1i = 1 / (gam - 1).
+template <bool NR = false, class St>
+__device__ __forceinline__ void flux_hlld_st(double* flux, const St& S, double bx, double gam, double gm1i,
+                                             unsigned& err) {
+  double wL[NM], wR[NM];
+#pragma unroll
+  for (int n = 0; n < NM; ++n) {
+    wL[n] = n == BX ? bx : S.L(n);
+    wR[n] = n == BX ? bx : S.R(n);
+  }
   const double bx2 = sqr(bx);
   // pieces of prim2cons / primcons2flux that the HLL average needs
   const double b2L = bx2 + sqr(wL[BY]) + sqr(wL[BZ]);
@@ -443,7 +457,7 @@ __device__ __forceinline__ void flux_hlld(double* flux, const double* wL, const 
   const bool left = r <= 3;
   double w[NM];
 #pragma unroll
-  for (int n = 0; n < NM; ++n) w[n] = left ? wL[n] : wR[n];
+  for (int n = 0; n < NM; ++n) w[n] = n == BX ? bx : S.at(left, n);
   const double s_o = left ? sL : sR;          // outer wave
   const double s_i = left ? sLs : sRs;        // Alfven wave
   const double x = left ? xL : xR;
@@ -457,7 +471,7 @@ __device__ __forceinline__ void flux_hlld(double* flux, const double* wL, const 
   const double srs = left ? sqrt_rhoLs : sqrt_rhoRs;
 
   double u[NM], f[NM];
-  prim2cons(u, w, gam);
+  prim2cons_g(u, w, gm1i);
   primcons2flux(f, w, u);
   // single-star state (fluxes_c.c:690-760)
   double es = (svx * u[EN] - pt * w[VX] + pts * sM + bx * (w[VX] * bx + w[VY] * w[BY] + w[VZ] * w[BZ] - vsbs)) * sMi;
@@ -476,6 +490,21 @@ __device__ __forceinline__ void flux_hlld(double* flux, const double* wL, const 
     flux[n] = v;
   }
   flux[BX] = 0.;
+}
+
+// face states held in registers
+struct FaceRegs {
+  const double* wL;
+  const double* wR;
+  __device__ __forceinline__ double L(int n) const { return wL[n]; }
+  __device__ __forceinline__ double R(int n) const { return wR[n]; }
+  __device__ __forceinline__ double at(bool left, int n) const { return left ? wL[n] : wR[n]; }
+};
+
+template <bool NR = false>
+__device__ __forceinline__ void flux_hlld(double* flux, const double* wL, const double* wR, double gam,
+                                          unsigned& err) {
+  flux_hlld_st<NR>(flux, FaceRegs{wL, wR}, wL[BX], gam, 1. / (gam - 1.), err);
 }
 
 // eos_c.h:100-216 prim2char (MHD): the differences vc (local sweep frame) in
@@ -604,6 +633,24 @@ __device__ __forceinline__ void riemann(double* flux, const double* wL, const do
   else if constexpr (RS == RS_HLLC) flux_hllc(flux, wL, wR, gam);
   else if constexpr (RS == RS_HLL_HYDRO) flux_hll_hydro(flux, wL, wR, gam);
   else flux_hll(flux, wL, wR, gam);
+}
+
+// The flux of a face whose states an accessor gives (as flux_hlld_st takes
+// them), with normal field bx.
+template <int RS, class St>
+__device__ __forceinline__ void face_flux(double* flux, const St& S, double bx, double gam, double gm1i,
+                                          unsigned& err) {
+  if constexpr (RS == RS_HLLD) {
+    flux_hlld_st<true>(flux, S, bx, gam, gm1i, err);
+  } else {
+    double wL[NM], wR[NM];
+#pragma unroll
+    for (int n = 0; n < NM; ++n) {
+      wL[n] = n == BX ? bx : S.L(n);
+      wR[n] = n == BX ? bx : S.R(n);
+    }
+    riemann<RS, true>(flux, wL, wR, gam, err);
+  }
 }
 
 // reconstr_c.h:28-44

@@ -18,6 +18,7 @@ namespace BNZ_NS {
 #include "bnz_bc_dt.cuh"
 #include "bnz_diffusion.cuh"
 #include "bnz_source.cuh"
+#include "bnz_split_flux.cuh"
 #include "bnz_split.cuh"
 #include "bnz_fused.cuh"
 #include "bnz_fused3d.cuh"
@@ -263,129 +264,107 @@ inline dim3 cell_grid(const plain::Box& b) {
   return dim3((b.hi.x - b.lo.x + 32) / 32, (b.hi.y - b.lo.y + 8) / 8, (b.hi.z - b.lo.z + kz) / kz);
 }
 
-// The prim arrays a split stage reads: w on [vlo, vhi], wfb elsewhere.
-struct SplitSrc {
-  const double* w;
-  const double* wfb;
-  int3 vlo, vhi;
-};
+// Walk length of a column walk: the faces a thread walks, so that the launch
+// holds about four times the blocks the device keeps resident (an even last
+// wave), at least `least` faces (a PLM walk starts with a slope that its
+// neighbour forms too: one in four at most) and at most 32.
+inline int walk_len(long long units, long long blocks_per_unit_row, int resident, int least) {
+  const long long want = 4LL * resident;  // blocks
+  long long parts = (want + blocks_per_unit_row - 1) / std::max(1LL, blocks_per_unit_row);
+  parts = std::max(parts, (units + 31) / 32);
+  parts = std::min(parts, std::max(1LL, units / least));
+  return (int)((units + parts - 1) / parts);
+}
 
-// The corrector's PLM fluxes of a 3D grid with tensor maps: a persistent
-// kernel of two blocks per SM (at most one per tile), each tile one TMA box of
-// the predictor's prim (x sweep: first face column even).
-template <int AX, int RS>
-void launch_flux_tma(const StepArgs& a, const SplitSrc& s, const double* bf, const plain::Box& b, unsigned nblk) {
-  constexpr size_t sm = sizeof(split::FluxSmem<AX>);
-  static bool attr = false;  // once per kernel
-  if (!attr) {
-    cudaFuncSetAttribute(split::k_flux_tile_tma<AX, RS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    attr = true;
+// Resident blocks of a kernel on the whole device (asked for once per kernel).
+template <class K>
+int flux_resident(K kernel, int smem, int& cache) {
+  if (!cache) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    int n = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, split::FLUX_NT, smem);
+    cache = std::max(1, n);
   }
-  split::k_flux_tile_tma<AX, RS><<<nblk, 256, sm, a.stream>>>(a.g, a.smaps, s.wfb, s.vlo, s.vhi, bf, a.flx[AX], b,
-                                                              a.limiter, a.charact_proj, a.err);
+  return cache * sm_count();
+}
+
+template <int AX, int ORDER, int RS, int CP>
+void launch_split_flux(const StepArgs& a, const double* w, const double* bf, const plain::Box& b) {
+  static int per_sm = 0;
+  const long long nx = b.hi.x - b.lo.x + 1, ny = b.hi.y - b.lo.y + 1, nz = b.hi.z - b.lo.z + 1;
+  constexpr int NT = split::FLUX_NT;
+  if constexpr (AX == 0) {
+    constexpr int sm = split::RowSmem<ORDER, CP>::BYTES, step = ORDER ? 31 : 32;
+    const int res = flux_resident(split::k_flux_row<ORDER, RS, CP>, sm, per_sm);
+    const long long nent = (nx + 1 + 2 * ORDER) * ny * nz, nseg = (nent + step - 1) / step;
+    // a row of units: one segment for each warp of the device
+    const int len = (int)std::max(1LL, std::min(32LL, nseg / (4LL * res * (NT / 32))));
+    const long long nwarp = (nseg + len - 1) / len;
+    split::k_flux_row<ORDER, RS, CP><<<(unsigned)((nwarp + NT / 32 - 1) / (NT / 32)), NT, sm, a.stream>>>(
+        a.g, w, bf, a.flx[0], b, a.limiter, len, a.err);
+  } else {
+    constexpr int sm = split::ColSmem<ORDER, CP>::BYTES;
+    const int res = flux_resident(split::k_flux_march<AX, ORDER, RS, CP>, sm, per_sm);
+    const long long nf = AX == 1 ? ny : nz, ncol = nx * (AX == 1 ? nz : ny), nbx = (ncol + NT - 1) / NT;
+    const int len = walk_len(nf, nbx, res, 4);
+    split::k_flux_march<AX, ORDER, RS, CP><<<dim3((unsigned)nbx, (unsigned)((nf + len - 1) / len)), NT, sm, a.stream>>>(
+        a.g, w, bf, a.flx[AX], b, a.limiter, len, a.err);
+  }
+}
+
+template <int AX, int ORDER, int CP>
+void launch_split_flux(const StepArgs& a, const double* w, const double* bf, const plain::Box& b) {
+  switch (a.rsolver) {
+    case dev::RS_HLLD: launch_split_flux<AX, ORDER, dev::RS_HLLD, CP>(a, w, bf, b); break;
+    case dev::RS_HLLT: launch_split_flux<AX, ORDER, dev::RS_HLLT, CP>(a, w, bf, b); break;
+    case dev::RS_HLLC: launch_split_flux<AX, ORDER, dev::RS_HLLC, CP>(a, w, bf, b); break;
+    case dev::RS_HLL_HYDRO: launch_split_flux<AX, ORDER, dev::RS_HLL_HYDRO, CP>(a, w, bf, b); break;
+    default: launch_split_flux<AX, ORDER, dev::RS_HLL, CP>(a, w, bf, b); break;
+  }
 }
 
 template <int AX>
-int split_flux_tma(const StepArgs& a, const SplitSrc& s, const double* bf, const plain::Box& b) {
-  using T = split::FTT<AX>;
-  const int lo[3] = {b.lo.x, b.lo.y, b.lo.z}, hi[3] = {b.hi.x, b.hi.y, b.hi.z};
-  const int lb0 = AX == 0 ? lo[T::TAX] : (lo[T::TAX] & ~1);
-  const long long na = (hi[AX] - lo[AX] + T::NA) / T::NA, nb = (hi[T::TAX] - lb0 + T::NB) / T::NB;
-  const long long ntile = na * nb * (hi[T::OAX] - lo[T::OAX] + 1);
-  const unsigned nblk = (unsigned)std::min<long long>(ntile, 2LL * sm_count());
-  switch (a.rsolver) {
-    case dev::RS_HLLD: launch_flux_tma<AX, dev::RS_HLLD>(a, s, bf, b, nblk); break;
-    case dev::RS_HLLT: launch_flux_tma<AX, dev::RS_HLLT>(a, s, bf, b, nblk); break;
-    case dev::RS_HLLC: launch_flux_tma<AX, dev::RS_HLLC>(a, s, bf, b, nblk); break;
-    case dev::RS_HLL_HYDRO: launch_flux_tma<AX, dev::RS_HLL_HYDRO>(a, s, bf, b, nblk); break;
-    default: launch_flux_tma<AX, dev::RS_HLL>(a, s, bf, b, nblk); break;
-  }
+int split_flux(const StepArgs& a, int order, const double* w, const double* bf, const plain::Box& b) {
+  if (order == 0) launch_split_flux<AX, 0, 0>(a, w, bf, b);
+  else if (a.charact_proj) launch_split_flux<AX, 1, 1>(a, w, bf, b);
+  else launch_split_flux<AX, 1, 0>(a, w, bf, b);
   return 1;
 }
 
-template <int AX, int ORDER>
-int split_flux(const StepArgs& a, const SplitSrc& s, const double* bf, const plain::Box& b) {
-  using T = split::FT<AX>;
-  if (ORDER == 1 && a.g.dims == 3 && a.smaps && s.w == a.cons_s && (AX != 0 || (b.lo.x & 1) == 0))
-    return split_flux_tma<AX>(a, s, bf, b);
-  const int lo[3] = {b.lo.x, b.lo.y, b.lo.z}, hi[3] = {b.hi.x, b.hi.y, b.hi.z};
-  const long long na = (hi[AX] - lo[AX] + T::NA) / T::NA, nb = (hi[T::TAX] - lo[T::TAX] + T::NB) / T::NB;
-  const unsigned nblk = (unsigned)(na * nb * (hi[T::OAX] - lo[T::OAX] + 1));
-  switch (a.rsolver) {
-    case dev::RS_HLLD:
-      split::k_flux_tile<AX, ORDER, dev::RS_HLLD><<<nblk, T::NT, 0, a.stream>>>(
-          a.g, s.w, s.wfb, s.vlo, s.vhi, bf, a.flx[AX], b, a.limiter, a.charact_proj, a.err);
-      break;
-    case dev::RS_HLLT:
-      split::k_flux_tile<AX, ORDER, dev::RS_HLLT><<<nblk, T::NT, 0, a.stream>>>(
-          a.g, s.w, s.wfb, s.vlo, s.vhi, bf, a.flx[AX], b, a.limiter, a.charact_proj, a.err);
-      break;
-    case dev::RS_HLLC:
-      split::k_flux_tile<AX, ORDER, dev::RS_HLLC><<<nblk, T::NT, 0, a.stream>>>(
-          a.g, s.w, s.wfb, s.vlo, s.vhi, bf, a.flx[AX], b, a.limiter, a.charact_proj, a.err);
-      break;
-    case dev::RS_HLL_HYDRO:
-      split::k_flux_tile<AX, ORDER, dev::RS_HLL_HYDRO><<<nblk, T::NT, 0, a.stream>>>(
-          a.g, s.w, s.wfb, s.vlo, s.vhi, bf, a.flx[AX], b, a.limiter, a.charact_proj, a.err);
-      break;
-    default:
-      split::k_flux_tile<AX, ORDER, dev::RS_HLL><<<nblk, T::NT, 0, a.stream>>>(
-          a.g, s.w, s.wfb, s.vlo, s.vhi, bf, a.flx[AX], b, a.limiter, a.charact_proj, a.err);
-      break;
-  }
-  return 1;
-}
-
-// Donor-cell fluxes from one prim array go through plain::k_flux: with no
-// slopes to share, staging the cells in shared memory only adds a barrier
-// (the split tile kernel measured about 9 % slower there).
-template <int AX>
-int split_flux(const StepArgs& a, int order, const SplitSrc& s, const double* bf, const plain::Box& b) {
-  if (order == 0 && s.w == s.wfb) return launch_flux<AX>(a, 0, s.w, bf, b);
-  return order == 0 ? split_flux<AX, 0>(a, s, bf, b) : split_flux<AX, 1>(a, s, bf, b);
-}
-
-// One VL2 stage on the split path (vanleer.pyx:104-120 or 130-151): the face
-// fluxes over the boxes of integrate_hydro, the edge EMFs over the box of
-// integrate_field, then the fused update of the stage's range from U^n =
-// prim2cons(a.prim) into w1.
-int split_stage(const StepArgs& a, const SplitSrc& s, double* w1, double* b1, const double* b0, double* bsave,
-                const double* bf, int order, const double* dtp, double fac) {
+// One VL2 stage on the split path (vanleer.pyx:104-120 or 130-151) on the
+// cells of `b`: the fluxes of their faces and of the faces one cell beside
+// them, the edge EMFs, then the fused update from U^n = prim2cons(a.prim) into
+// w1.  w: the stage input's prim.
+int split_stage(const StepArgs& a, const plain::Box& b, const double* w, double* w1, double* b1, const double* b0,
+                double* bsave, const double* bf, int order, const double* dtp, double fac) {
   const GridDev& g = a.g;
-  int l[6];
-  integr_lims(g, order, l);
-  const int il = l[0], iu = l[1], jl = l[2], ju = l[3], kl = l[4], ku = l[5];
+  const int il = b.lo.x, iu = b.hi.x, jl = b.lo.y, ju = b.hi.y, kl = b.lo.z, ku = b.hi.z;
   const int jb = g.dims >= 2 ? jl - 1 : 0, je = g.dims >= 2 ? ju + 1 : 0;
   const int kb = g.dims >= 3 ? kl - 1 : 0, ke = g.dims >= 3 ? ku + 1 : 0;
-  int nl = split_flux<0>(a, order, s, bf, mkbox(il, iu + 1, jb, je, kb, ke));
-  if (g.dims >= 2) nl += split_flux<1>(a, order, s, bf, mkbox(il - 1, iu + 1, jl, ju + 1, kb, ke));
-  if (g.dims >= 3) nl += split_flux<2>(a, order, s, bf, mkbox(il - 1, iu + 1, jl - 1, ju + 1, kl, ku + 1));
+  int nl = split_flux<0>(a, order, w, bf, mkbox(il, iu + 1, jb, je, kb, ke));
+  if (g.dims >= 2) nl += split_flux<1>(a, order, w, bf, mkbox(il - 1, iu + 1, jl, ju + 1, kb, ke));
+  if (g.dims >= 3) nl += split_flux<2>(a, order, w, bf, mkbox(il - 1, iu + 1, jl - 1, ju + 1, kl, ku + 1));
   {
-    plain::Box b = mkbox(il, iu + 1, jl, g.dims >= 2 ? ju + 1 : 0, kl, g.dims >= 3 ? ku + 1 : 0);
-    split::k_ee<<<cell_grid(b), dim3(32, 8), 0, a.stream>>>(g, s.w, s.wfb, s.vlo, s.vhi, a.flx[0], a.flx[1],
-                                                             a.flx[2], a.ee, b);
+    plain::Box be = mkbox(il, iu + 1, jl, g.dims >= 2 ? ju + 1 : 0, kl, g.dims >= 3 ? ku + 1 : 0);
+    split::k_ee<<<cell_grid(be), dim3(32, 8), 0, a.stream>>>(g, w, a.flx[0], a.flx[1], a.flx[2], a.ee, be);
   }
-  plain::Box b = mkbox(il, iu, jl, ju, kl, ku);
   if (g.dims == 3 && a.smaps) {
-    // the TMA-fed form (3D, even Ntot_x): blocks of 32 x 8 columns from an
-    // even first column, split::UPD_KZ planes each
+    // the TMA-fed form (3D, even Ntot_x): blocks of 32 x 8 columns,
+    // split::UPD_KZ planes each
     constexpr size_t sm = sizeof(split::TmaSmem);
     static bool attr = false;  // once per floating-point build
     if (!attr) {
       cudaFuncSetAttribute(split::k_update_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
       attr = true;
     }
-    const int x0base = b.lo.x & ~1;
-    const dim3 grid((b.hi.x - x0base + 32) / 32, (b.hi.y - b.lo.y + 8) / 8,
-                    (b.hi.z - b.lo.z + split::UPD_KZ) / split::UPD_KZ);
     const int b0map = b0 == a.bfld ? split::TM_BFLD : split::TM_BSAVE;
-    split::k_update_tma<<<grid, dim3(32, 8), sm, a.stream>>>(g, w1, s.w, b1, bsave, a.smaps, b0map, b, x0base, dtp,
-                                                             fac, a.src, a.grav[0], a.grav[1], a.grav[2], a.fdriv,
-                                                             a.err);
+    split::k_update_tma<<<cell_grid(b), dim3(32, 8), sm, a.stream>>>(g, w1, w, b1, bsave, a.smaps, b0map, b, dtp, fac,
+                                                                     a.src, a.grav[0], a.grav[1], a.grav[2], a.fdriv,
+                                                                     a.err);
     return nl + 2;
   }
   split::k_update<<<cell_grid(b), dim3(32, 8), 0, a.stream>>>(
-      g, w1, a.prim, s.w, b1, b0, bsave, a.flx[0], a.flx[1], a.flx[2], a.ee, b, dtp, fac, a.src, a.grav[0],
+      g, w1, a.prim, w, b1, b0, bsave, a.flx[0], a.flx[1], a.flx[2], a.ee, b, dtp, fac, a.src, a.grav[0],
       a.grav[1], a.grav[2], a.fdriv, a.err);
   return nl + 2;
 }
@@ -393,27 +372,24 @@ int split_stage(const StepArgs& a, const SplitSrc& s, double* w1, double* b1, co
 
 // vanleer.pyx:101-151 on the split path.  The predictor writes W^(n+1/2) to
 // a.cons_s (cells 1..Ntot-2 of each active axis), so that a.prim keeps W^n for
-// the corrector's U^n; the corrector reads W^(n+1/2) there and W^n on the
-// outer cells, as the plain path's in-place prim holds them.  The predictor
-// also saves the faces of b^n it reads into the spare face array a.ec (the
-// split path forms the cell EMFs on the fly), so that the corrector can
-// update a.bfld in place of a neighbour's reads: it reads b^n from the copy.
-// The conserved state is not written: the context forms it from prim after
-// the boundary fill, when it is asked for.  In the hydro build (field entries
-// and face field held at zero, the hydro solvers' field fluxes zero) the same
-// launches run and the field stays zero.
+// the corrector's U^n.  The corrector updates the active cells, which read no
+// cell the predictor did not write; the reference's one more ring of cells
+// (integrator.pyx:375-383) is overwritten by the boundary fill that follows.
+// The predictor also saves the faces of b^n it reads into the spare face array
+// a.ec (the split path forms the cell EMFs on the fly), so that the corrector
+// can update a.bfld in place of a neighbour's reads: it reads b^n from the
+// copy.  The conserved state is not written: the context forms it from prim
+// after the boundary fill, when it is asked for.  In the hydro build (field
+// entries and face field held at zero, the hydro solvers' field fluxes zero)
+// the same launches run and the field stays zero.
 int split_predictor_corrector(const StepArgs& a, const double* dtp) {
   const GridDev& g = a.g;
-  const int N[3] = {g.nx, g.ny, g.nz};
-  int lo[3], hi[3];
-  for (int d = 0; d < 3; ++d) {
-    lo[d] = d < g.dims ? 1 : 0;
-    hi[d] = d < g.dims ? N[d] - 2 : 0;
-  }
-  const SplitSrc pred = {a.prim, a.prim, make_int3(0, 0, 0), make_int3(g.nx - 1, g.ny - 1, g.nz - 1)};
-  const SplitSrc corr = {a.cons_s, a.prim, make_int3(lo[0], lo[1], lo[2]), make_int3(hi[0], hi[1], hi[2])};
-  int nl = split_stage(a, pred, a.cons_s, a.bfld_s, a.bfld, a.ec, a.bfld, 0, dtp, 0.5);
-  nl += split_stage(a, corr, a.prim, a.bfld, a.ec, nullptr, a.bfld_s, a.reconstr_order, dtp, 1.0);
+  int l[6];
+  integr_lims(g, 0, l);
+  const plain::Box pred = mkbox(l[0], l[1], l[2], l[3], l[4], l[5]);
+  const plain::Box act = mkbox(g.i1, g.i2, g.j1, g.j2, g.k1, g.k2);
+  int nl = split_stage(a, pred, a.prim, a.cons_s, a.bfld_s, a.bfld, a.ec, a.bfld, 0, dtp, 0.5);
+  nl += split_stage(a, act, a.cons_s, a.prim, a.bfld, a.ec, nullptr, a.bfld_s, a.reconstr_order, dtp, 1.0);
   return nl;
 }
 

@@ -4,11 +4,9 @@
 // Where the plain path (bnz_plain.cuh) follows the reference loop by loop, the
 // split path keeps its decomposition (fluxes and edge EMFs through HBM) and
 // removes its costs:
-//   * k_flux_tile: a block stages a pencil tile of cells (NB lines of NA faces
-//     along the sweep axis, with the two-cell halo) in shared memory and forms
-//     every cell's PLM half slopes once (reconstr_c.c:54-91), where
-//     plain::k_flux forms both one-sided slopes of every face itself (the
-//     donor-cell predictor, with no slopes to share, keeps plain::k_flux);
+//   * the flux kernels (bnz_split_flux.cuh) load every cell once and form its
+//     PLM half slopes once (reconstr_c.c:54-91), where plain::k_flux forms both
+//     one-sided slopes of every face itself;
 //   * k_ee forms the cell-centred EMF (ct.pyx:128-148) of the cells it needs
 //     on the fly instead of reading a separate array;
 //   * k_update: per cell, prim2cons of the step's input, the conservative
@@ -17,172 +15,16 @@
 //     (integrator.pyx:132-170) and cons2prim (eos.pyx:13-44) in one pass,
 //     where the plain path runs up to eight launches and keeps a conserved
 //     state in HBM between them.
-// A face is formed by exactly one block and no kernel waits on a barrier
+// A face is formed by exactly one thread and no kernel waits on a barrier
 // between Riemann solves (what bounds the z-marching chunk kernels).  Every
 // expression is the plain path's, so the exact build is bitwise equal to it
 // and to the oracle (the fast build's van Leer limiter differs: see
 // half_slope_split).  The hydro build runs the same launches on zero fields.
-// Included inside the per-floating-point-mode namespace, after bnz_plain.cuh
-// and bnz_source.cuh.
+// Included inside the per-floating-point-mode namespace, after bnz_plain.cuh,
+// bnz_source.cuh and bnz_split_flux.cuh.
 #pragma once
 
 namespace split {
-
-using namespace dev;
-
-// slope slot of variable n (the normal field has none)
-__device__ __forceinline__ constexpr int slot8(int n) { return n < BX ? n : n - 1; }
-
-// Pencil tiles of the flux kernel of axis AX: NA faces along AX on each of NB
-// lines along the transverse axis TAX (y for the x sweep, x for the y and z
-// sweeps, so that a warp's loads and stores run along x); OAX is the axis the
-// block index walks one line at a time.  (NA + 1) NB = 256 threads: one slope
-// cell per thread.  Shared arrays are laid out with x fastest, which keeps a
-// warp's accesses on distinct banks.
-template <int AX>
-struct FT {
-  static constexpr int NA = AX == 0 ? 31 : 15;
-  static constexpr int NB = AX == 0 ? 8 : 16;
-  static constexpr int TAX = AX == 0 ? 1 : 0;
-  static constexpr int OAX = AX == 2 ? 1 : 2;
-  static constexpr int NS = NA + 3;             // staged cells along AX
-  static constexpr int NT = (NA + 1) * NB;
-  static constexpr int DA = AX == 0 ? 1 : NB;   // stride along AX (staged cells and slopes)
-  static constexpr int WN = NB * NS;            // stride between staged fields
-  __device__ static constexpr int ws(int n, int sa, int lb) {  // staged cell sa of line lb
-    return AX == 0 ? (n * NB + lb) * NS + sa : (n * NS + sa) * NB + lb;
-  }
-  __device__ static constexpr int ds(int s, int la, int lb) {  // slope of cell la of line lb
-    return AX == 0 ? (s * NB + lb) * (NA + 1) + la : (s * (NA + 1) + la) * NB + lb;
-  }
-  static_assert(NT == 256, "one slope cell per thread");
-};
-
-__device__ __forceinline__ int ax_of(int3 v, int a) { return a == 0 ? v.x : a == 1 ? v.y : v.z; }
-
-// reconstr_c.c:54-91 half slope; in the fast build the van Leer limiter's
-// quotient 2ab/(a+b) is 2ab times the Newton-refined reciprocal of a + b
-// (bnz_fastmath.cuh: within 2 ulp; ab > 0 makes a and b one-signed, so
-// |a + b| >= 2 sqrt(ab) is a normal number)
-template <int LIM>
-__device__ __forceinline__ double half_slope_split(double wm, double wc, double wp) {
-#if BNZ_FAST_MATH
-  if (LIM == LIM_VL) {
-    const double a = wc - wm, b = wp - wc, ab = a * b;
-    return 0.5 * ((ab > 0.) ? (2. * ab) * bnz_nr_rcp(a + b) : 0.);
-  }
-#endif
-  return half_slope<LIM>(wm, wc, wp);
-}
-
-// the eight half slopes (all but the normal field) of the staged cell at p
-// into the slope table, one limiter for the whole loop
-template <int LIM, class T>
-__device__ __forceinline__ void cell_slopes(const double* p, double* sD, int la, int lb) {
-#pragma unroll
-  for (int n = 0; n < NM; ++n) {
-    if (n == BX) continue;
-    sD[T::ds(slot8(n), la, lb)] = half_slope_split<LIM>(p[n * T::WN - T::DA], p[n * T::WN], p[n * T::WN + T::DA]);
-  }
-}
-
-// Fluxes of the AX faces of `box` (face index along AX = the cell on its
-// right), in the global variable order as plain::k_flux stores them (the
-// normal field entry, which nothing reads, is not stored).  ORDER 0: donor
-// cell (reconstr_c.c:8-22); ORDER 1: PLM with limiter lim (reconstr_c.c:29-91),
-// in characteristic variables when cp.  Normal field from the face array.
-// Cells outside [vlo, vhi] are read from wfb instead of w (the corrector reads
-// the predictor's output, which covers cells 1..Ntot-2 of each active axis,
-// and the step's input prim elsewhere).
-template <int AX, int ORDER, int RS>
-__global__ void __launch_bounds__(256, 2) k_flux_tile(GridDev g, const double* __restrict__ w,
-                                                      const double* __restrict__ wfb, int3 vlo, int3 vhi,
-                                                      const double* __restrict__ bf, double* __restrict__ F,
-                                                      plain::Box box, int lim, int cp, unsigned* err) {
-  using T = FT<AX>;
-  constexpr int NA = T::NA, NB = T::NB, NS = T::NS, DA = T::DA, WN = T::WN;
-  __shared__ double sW[NM * WN];
-  __shared__ double sD[ORDER ? 8 * NB * (NA + 1) : 1];
-  const int lo_a = ax_of(box.lo, AX), hi_a = ax_of(box.hi, AX);
-  const int lo_b = ax_of(box.lo, T::TAX), hi_b = ax_of(box.hi, T::TAX);
-  const int na = (hi_a - lo_a + NA) / NA, nb = (hi_b - lo_b + NB) / NB;
-  const int ta = blockIdx.x % na, tb = (blockIdx.x / na) % nb, to = blockIdx.x / (na * nb);
-  const int a0 = lo_a + ta * NA, b0 = lo_b + tb * NB, o = ax_of(box.lo, T::OAX) + to;
-  const long long st[3] = {1, (long long)g.nx, (long long)g.nx * g.ny};
-  const int N[3] = {g.nx, g.ny, g.nz};
-  const long long sa = st[AX], sb = st[T::TAX], so = st[T::OAX];
-  // stage cells a0-2 .. a0+NA of the NB lines, in the sweep frame's variable
-  // order; cells outside the array are neither loaded nor used
-  for (int t = threadIdx.x; t < NS * NB; t += T::NT) {
-    const int ia = AX == 0 ? t % NS : t / NB;
-    const int ib = AX == 0 ? t / NS : t % NB;
-    const int a = a0 - 2 + ia, b = b0 + ib;
-    if (a < 0 || a >= N[AX] || b > hi_b) continue;
-    const long long c = a * sa + b * sb + o * so;
-    const bool in = a >= ax_of(vlo, AX) && a <= ax_of(vhi, AX) && b >= ax_of(vlo, T::TAX) &&
-                    b <= ax_of(vhi, T::TAX) && o >= ax_of(vlo, T::OAX) && o <= ax_of(vhi, T::OAX);
-    const double* src = in ? w : wfb;
-#pragma unroll
-    for (int n = 0; n < NM; ++n) sW[T::ws(n, ia, ib)] = src[plain::perm<AX>(n) * g.sv + c];
-  }
-  __syncthreads();
-  const int la = AX == 0 ? threadIdx.x % (NA + 1) : threadIdx.x / NB;
-  const int lb = AX == 0 ? threadIdx.x / (NA + 1) : threadIdx.x % NB;
-  if (ORDER == 1) {
-    // the half slope of cell a0-1+la (staged index la+1), once per cell
-    const int a = a0 - 1 + la;
-    if (a >= 1 && a + 1 < N[AX] && a <= hi_a && b0 + lb <= hi_b) {
-      const double* p = sW + T::ws(0, la + 1, lb);
-      if (cp) {
-        double wm[NM], wc[NM], wp[NM], d[NM];
-#pragma unroll
-        for (int n = 0; n < NM; ++n) {
-          wm[n] = p[n * WN - DA];
-          wc[n] = p[n * WN];
-          wp[n] = p[n * WN + DA];
-        }
-        plain::half_slopes_char_rt(lim, wm, wc, wp, g.gam, d);
-#pragma unroll
-        for (int n = 0; n < NM; ++n)
-          if (n != BX) sD[T::ds(slot8(n), la, lb)] = d[n];
-      } else if (lim == LIM_MC) {
-        cell_slopes<LIM_MC, T>(p, sD, la, lb);
-      } else if (lim == LIM_MM) {
-        cell_slopes<LIM_MM, T>(p, sD, la, lb);
-      } else {
-        cell_slopes<LIM_VL, T>(p, sD, la, lb);
-      }
-    }
-    __syncthreads();
-  }
-  // the face a0+la between cells a0+la-1 and a0+la (threads la == NA have none)
-  const int f = a0 + la, b = b0 + lb;
-  if (la >= NA || f > hi_a || b > hi_b) return;
-  const long long c = f * sa + b * sb + o * so;
-  const double* p = sW + T::ws(0, la + 2, lb);  // staged cell f
-  double wL[NM], wR[NM];
-#pragma unroll
-  for (int n = 0; n < NM; ++n) {
-    if (n == BX) continue;
-    if (ORDER == 0) {
-      wL[n] = p[n * WN - DA];
-      wR[n] = p[n * WN];
-    } else {
-      wL[n] = p[n * WN - DA] + sD[T::ds(slot8(n), la, lb)];
-      wR[n] = p[n * WN] - sD[T::ds(slot8(n), la + 1, lb)];
-    }
-  }
-  const double bx = bf[AX * g.sv + c];
-  wL[BX] = bx;
-  wR[BX] = bx;
-  unsigned e = 0;
-  double fl[NM];
-  riemann<RS, true>(fl, wL, wR, g.gam, e);
-#pragma unroll
-  for (int n = 0; n < NM; ++n)
-    if (n != BX) F[plain::perm<AX>(n) * g.sv + c] = fl[n];
-  if (e) atomicOr(err, e);
-}
 
 // k_ee and k_update: a thread walks UPD_KZ cells up z (blocks of 32 x 8
 // columns) and asks L2 for the inputs of the cell two planes ahead while it
@@ -203,10 +45,10 @@ __device__ __forceinline__ double ec_at(const double* __restrict__ w, long long 
 }
 
 // ct.pyx:153-215 (interp_ee1): plain::k_ee with the cell EMFs formed from the
-// stage input prim: w on [vlo, vhi], wfb elsewhere (as in k_flux_tile)
-__global__ void k_ee(GridDev g, const double* __restrict__ w_in, const double* __restrict__ wfb, int3 vlo,
-                     int3 vhi, const double* __restrict__ fx, const double* __restrict__ fy,
-                     const double* __restrict__ fz, double* __restrict__ ee, plain::Box box) {
+// stage input prim
+__global__ void k_ee(GridDev g, const double* __restrict__ w_in, const double* __restrict__ fx,
+                     const double* __restrict__ fy, const double* __restrict__ fz, double* __restrict__ ee,
+                     plain::Box box) {
   const long long sv = g.sv, sy = g.nx, sz = (long long)g.nx * g.ny;
   const int i = box.lo.x + (int)(blockIdx.x * 32 + threadIdx.x);
   const int j = box.lo.y + (int)(blockIdx.y * 8 + threadIdx.y);
@@ -231,29 +73,24 @@ __global__ void k_ee(GridDev g, const double* __restrict__ w_in, const double* _
       prefetch_l2(fz + BY * sv + p);
       prefetch_l2(fz + BY * sv + p - sy);
     }
-    // the source array of the cell (i - di, j - dj, k - dk)
-    auto W = [&](int di, int dj, int dk) {
-      const int x = i - di, y = j - dj, z = k - dk;
-      return x >= vlo.x && x <= vhi.x && y >= vlo.y && y <= vhi.y && z >= vlo.z && z <= vhi.z ? w_in : wfb;
-    };
     if (g.dims == 3) {
       ee[c] = (0.5 * (-fy[BZ * sv + c - sz] - fy[BZ * sv + c] + fz[BY * sv + c - sy] + fz[BY * sv + c]) -
-               0.25 * (ec_at<0>(W(0, 1, 0), sv, c - sy) + ec_at<0>(W(0, 0, 0), sv, c) +
-                       ec_at<0>(W(0, 1, 1), sv, c - sz - sy) + ec_at<0>(W(0, 0, 1), sv, c - sz)));
+               0.25 * (ec_at<0>(w_in, sv, c - sy) + ec_at<0>(w_in, sv, c) +
+                       ec_at<0>(w_in, sv, c - sz - sy) + ec_at<0>(w_in, sv, c - sz)));
       ee[sv + c] = (0.5 * (-fz[BX * sv + c - 1] - fz[BX * sv + c] + fx[BZ * sv + c - sz] + fx[BZ * sv + c]) -
-                    0.25 * (ec_at<1>(W(1, 0, 0), sv, c - 1) + ec_at<1>(W(0, 0, 0), sv, c) +
-                            ec_at<1>(W(1, 0, 1), sv, c - sz - 1) + ec_at<1>(W(0, 0, 1), sv, c - sz)));
+                    0.25 * (ec_at<1>(w_in, sv, c - 1) + ec_at<1>(w_in, sv, c) +
+                            ec_at<1>(w_in, sv, c - sz - 1) + ec_at<1>(w_in, sv, c - sz)));
       ee[2 * sv + c] = (0.5 * (-fx[BY * sv + c - sy] - fx[BY * sv + c] + fy[BX * sv + c - 1] + fy[BX * sv + c]) -
-                        0.25 * (ec_at<2>(W(1, 0, 0), sv, c - 1) + ec_at<2>(W(0, 0, 0), sv, c) +
-                                ec_at<2>(W(1, 1, 0), sv, c - sy - 1) + ec_at<2>(W(0, 1, 0), sv, c - sy)));
+                        0.25 * (ec_at<2>(w_in, sv, c - 1) + ec_at<2>(w_in, sv, c) +
+                                ec_at<2>(w_in, sv, c - sy - 1) + ec_at<2>(w_in, sv, c - sy)));
     } else if (g.dims == 2) {
       ee[c] = -fy[BZ * sv + c];
       ee[sv + c] = fx[BZ * sv + c];
       ee[2 * sv + c] = (0.5 * (-fx[BY * sv + c - sy] - fx[BY * sv + c] + fy[BX * sv + c - 1] + fy[BX * sv + c]) -
-                        0.25 * (ec_at<2>(W(1, 0, 0), sv, c - 1) + ec_at<2>(W(0, 0, 0), sv, c) +
-                                ec_at<2>(W(1, 1, 0), sv, c - sy - 1) + ec_at<2>(W(0, 1, 0), sv, c - sy)));
+                        0.25 * (ec_at<2>(w_in, sv, c - 1) + ec_at<2>(w_in, sv, c) +
+                                ec_at<2>(w_in, sv, c - sy - 1) + ec_at<2>(w_in, sv, c - sy)));
     } else {
-      ee[c] = -ec_at<0>(W(0, 0, 0), sv, c);
+      ee[c] = -ec_at<0>(w_in, sv, c);
       ee[sv + c] = fx[BZ * sv + c];
       ee[2 * sv + c] = -fx[BY * sv + c];
     }
