@@ -152,8 +152,8 @@ struct FusedTile {
 // Variants of the fused kernels the autotuner chooses from: tile shape
 // (cells along x, y), whether the predictor stages its input cells in shared
 // memory, and whether the stages run as persistent TMA-fed kernels.  A batch
-// starts on variant 8 (persistent, 15 x 14), a single grid on variant 0
-// (32 x 8: fewer tiles, one wave on a 256^2 grid).
+// starts on variant 8 (persistent, 15 x 14), a single grid on the shape that
+// grid_variant picks.
 struct FusedVariant {
   int tx, ty, staged, persistent;
 };
@@ -179,6 +179,32 @@ inline bool fused_variant_built(int v, bool hlld) {
 
 constexpr int BATCH_DEFAULT_VARIANT = 8;
 
+// Strip walks (bnz_walk2d.cuh) instead of a variant's tiles, for a batch on its
+// default variant or a single grid, without characteristic slopes: from the
+// size where enough strips fill the device.  Measured, us a step, walks against
+// tiles: batches 0.94 M zones 441 / 423 (persistent tiles ahead), 3.2 M 1220 /
+// 1338, 4.8 M 1793 / 2018; single grids (whose tiles are not persistent) 384^2
+// 139 / 95, 512^2 146 / 151, 640^2 173 / 240, 1024^2 422 / 581.
+constexpr long long WALK_MIN_BATCH = 1500000, WALK_MIN_GRID = 250000;
+// Rows of a strip: as many as leave every SM's 12 warps five strips each (a
+// strip forms its lowest row's faces besides its own), 8 to 32.
+inline int walk_rows(long long zones, int nsm) {
+  const long long r = zones / (30LL * 12 * 5 * nsm);
+  return (int)(r < 8 ? 8 : r > 32 ? 32 : r);
+}
+// Tiles of a single grid below that size: the kernels end a phase in a barrier,
+// so a grid whose tiles fit one wave (two blocks an SM) wants tiles whose phases
+// take one round of the block's threads: 14 x 14.  Where those need a second
+// wave and 32 x 8 does not, 32 x 8.  Measured, us for 10 or 8 steps with three
+// grids in flight / of one grid alone, 32 x 8 against 14 x 14: 64^2 178 / 503
+// against 142 / 397, 201 x 150 875 / 888 against 770 / 780 (host steps), 256^2
+// 288 / 474 against 308 / 576, 300^2 404 / 708 against 404 / 614, 384^2 647 /
+// 848 against 665 / 846.
+inline int grid_variant(int n0, int n1, int nsm) {
+  const int t14 = ((n0 + 13) / 14) * ((n1 + 13) / 14), t32 = ((n0 + 31) / 32) * ((n1 + 7) / 8);
+  return t14 > 2 * nsm && t32 <= 2 * nsm ? 0 : 9;
+}
+
 // dt modes of the fused step
 enum { FDT_CFL = 0, FDT_EXPLICIT = 1, FDT_FIXED = 2 };
 
@@ -192,6 +218,7 @@ struct FusedLaunch {
   int ntB;
   int rsolver, limiter, charact_proj;
   int variant;
+  int walk;  // the tiles are strips of the walk kernels, whatever the variant
   double cour;
   int dt_mode;
   double dt_fixed;

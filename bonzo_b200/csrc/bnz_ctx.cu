@@ -350,6 +350,38 @@ void make_tiles_uniform(int inst, int N0, int N1, int ng, int tx, int ty, std::v
     }
 }
 
+// Strips of at most `cols` x `rows` positions of about equal widths and heights
+// over [lo, lo + n) of both axes.
+void make_strips(int inst, const int* lo, const int* n, int cols, int rows, std::vector<FusedTile>& out) {
+  const int ns[2] = {(n[0] + cols - 1) / cols, (n[1] + rows - 1) / rows};
+  for (int y = 0; y < ns[1]; ++y)
+    for (int x = 0; x < ns[0]; ++x) {
+      const int t[2] = {x, y};
+      int a[2], b[2];
+      for (int d = 0; d < 2; ++d) {
+        a[d] = lo[d] + (int)((long long)n[d] * t[d] / ns[d]);
+        b[d] = lo[d] + (int)((long long)n[d] * (t[d] + 1) / ns[d]);
+      }
+      out.push_back(FusedTile{inst, a[0], a[1], b[0] - a[0], b[1] - a[1], 0});
+    }
+}
+
+// One instance's strips for the walk kernels (bnz_walk2d.cuh): the predictor
+// range (cells 1 .. Ntot-2) or the active cells.
+void make_walk_strips(int inst, int N0, int N1, int ng, bool pred, int rows, std::vector<FusedTile>& out) {
+  const int a = pred ? 1 : ng, g = pred ? 2 * ng - 2 : 0;
+  const int lo[2] = {a, a}, n[2] = {N0 + g, N1 + g};
+  make_strips(inst, lo, n, 30, rows, out);
+}
+
+int device_sms() {
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1)
+    return 148;
+  return n;
+}
+
 FusedInst make_inst(const bnz_ctx* c) {
   FusedInst I;
   memset(&I, 0, sizeof I);
@@ -400,6 +432,7 @@ FusedLaunch fused_launch(const bnz_ctx* c, int dt_mode) {
   f.limiter = c->md.limiter;
   f.charact_proj = c->md.charact_proj;
   f.variant = c->variant;
+  f.walk = c->walk;
   f.cour = c->md.cour;
   f.dt_mode = dt_mode;
   f.dt_fixed = c->md.dt_fixed;
@@ -436,11 +469,19 @@ cudaError_t build_ctx3(bnz_ctx* c) {
 
 // (Re)build the single-grid tile lists for the context's variant.
 cudaError_t build_ctx_tiles(bnz_ctx* c) {
+  const int n0 = c->i2 - c->i1 + 1, n1 = c->j2 - c->j1 + 1;
+  const long long zones = (long long)n0 * n1;
+  c->walk = zones >= WALK_MIN_GRID && !c->md.charact_proj;
+  c->variant = grid_variant(n0, n1, device_sms());
   const FusedVariant& v = FUSED_VARIANTS[c->variant];
+  const int rows = walk_rows(zones, device_sms());
   std::vector<FusedTile> tiles;
-  make_tiles(0, c->i2 - c->i1 + 1, c->j2 - c->j1 + 1, c->ng, true, v.tx, v.ty, tiles);
+  if (c->walk) make_walk_strips(0, n0, n1, c->ng, true, rows, tiles);
+  else if (c->variant == 0) make_tiles(0, n0, n1, c->ng, true, v.tx, v.ty, tiles);
+  else make_tiles_uniform(0, n0, n1, c->ng, v.tx, v.ty, tiles);
   c->ntA = (int)tiles.size();
-  make_tiles(0, c->i2 - c->i1 + 1, c->j2 - c->j1 + 1, c->ng, false, v.tx, v.ty, tiles);
+  if (c->walk) make_walk_strips(0, n0, n1, c->ng, false, rows, tiles);
+  else make_tiles(0, n0, n1, c->ng, false, v.tx, v.ty, tiles);
   c->ntB = (int)tiles.size() - c->ntA;
   if (c->d_tiles) cudaFree(c->d_tiles);
   c->d_tiles = nullptr;
@@ -1172,6 +1213,7 @@ struct bnz_batch {
   long long graph_launches = 0;
   double h_tmax = 0.;
   int variant = 0;
+  bool walk = false;  // the tiles are strips of the walk kernels
   const Launchers* L = nullptr;
   std::string err;
   // first predictor / corrector tile of every instance (n + 1 entries)
@@ -1236,12 +1278,13 @@ FusedLaunch batch_launch(const bnz_batch* b, int dt_mode) {
   f.limiter = b->md.limiter;
   f.charact_proj = b->md.charact_proj;
   f.variant = b->variant;
+  f.walk = b->walk;
   f.cour = b->md.cour;
   f.dt_mode = dt_mode;
   f.dt_fixed = b->md.dt_fixed;
   f.err = b->ctx.empty() ? nullptr : b->ctx[0]->d_err;
   f.stream = b->stream;
-  if (FUSED_VARIANTS[b->variant].persistent && b->d_maps) {
+  if (FUSED_VARIANTS[b->variant].persistent && b->d_maps && !b->walk) {
     f.wsmaps = b->d_maps;
     f.queue = b->d_queue;
     f.withhold = b->withhold;
@@ -1365,15 +1408,27 @@ int batch_build_tiles(bnz_batch* b) {
   std::vector<FusedTile> tA, tB;
   b->offA.assign(1, 0);
   b->offB.assign(1, 0);
+  long long zones = 0;
+  for (const bnz_ctx* c : b->ctx) zones += (long long)(c->i2 - c->i1 + 1) * (c->j2 - c->j1 + 1);
+  // (the test switch withholds the tile kernels' TMA loads, so it keeps them)
+  b->walk = b->variant == BATCH_DEFAULT_VARIANT && !b->withhold && zones >= WALK_MIN_BATCH && !b->md.charact_proj;
+  const int rows = walk_rows(zones, device_sms());
   for (int q = 0; q < (int)b->ctx.size(); ++q) {
     const bnz_ctx* c = b->ctx[q];
+    if (b->walk) {
+      make_walk_strips(q, c->i2 - c->i1 + 1, c->j2 - c->j1 + 1, c->ng, true, rows, tA);
+      make_walk_strips(q, c->i2 - c->i1 + 1, c->j2 - c->j1 + 1, c->ng, false, rows, tB);
+      b->offA.push_back((int)tA.size());
+      b->offB.push_back((int)tB.size());
+      continue;
+    }
     if (v.persistent == 2) make_tiles_uniform(q, c->i2 - c->i1 + 1, c->j2 - c->j1 + 1, c->ng, v.tx, v.ty, tA);
     else make_tiles(q, c->i2 - c->i1 + 1, c->j2 - c->j1 + 1, c->ng, true, v.tx, v.ty, tA);
     make_tiles(q, c->i2 - c->i1 + 1, c->j2 - c->j1 + 1, c->ng, false, v.tx, v.ty, tB);
     b->offA.push_back((int)tA.size());
     b->offB.push_back((int)tB.size());
   }
-  if (v.persistent) {
+  if (v.persistent && !b->walk) {
     static_assert(sizeof(CUtensorMap) == 128, "tensor maps are 128 bytes");
     // 6 maps per instance (TmaBox<tx, ty> in bnz_fused.cuh): ws with tx + 4
     // cells from an even column and ty + 4 rows; w[0], w[1] (9 fields) and
@@ -1399,7 +1454,7 @@ int batch_build_tiles(bnz_batch* b) {
     CKB(cudaMemcpy(b->d_maps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice));
     CKB(cudaMemset(b->d_queue, 0, 2 * sizeof(unsigned)));
   }
-  if (v.persistent == 2) {
+  if (v.persistent == 2 && !b->walk) {
     // predictor: boxes of TmaBoxP<tx, ty> over w[0], w[1] (9 fields) and
     // b[0], b[1] (3 faces): tx + 2 cells from an even column, ty + 2 rows;
     // only full interior tiles use them
@@ -2047,7 +2102,9 @@ int bnz_batch_step_host(bnz_batch* b, double* const* prim, double* const* bfld, 
 int bnz_batch_test_withhold_loads(bnz_batch* b, int on) {
   if (!b) return BNZ_ERR_ARG;
   CKB(cudaStreamSynchronize(b->stream));
+  const int before = b->withhold;
   b->withhold = on ? 1 : 0;
+  if (!b->dims3 && before != b->withhold) return batch_build_tiles(b);  // (drops the graph)
   if (b->graph) {  // a captured step holds the old value
     cudaGraphExecDestroy(b->graph);
     b->graph = nullptr;

@@ -715,13 +715,13 @@ __global__ void __launch_bounds__(256, 2) k_pred2d(const Inst* __restrict__ inst
   (void)lim;
 }
 
-__device__ __forceinline__ void copy_tile(const Inst& I, const Tile& T, int parity) {
+__device__ __forceinline__ void copy_tile(const Inst& I, const Tile& T, int parity, int tid, int nthreads) {
   const int i2 = I.ng + I.N[0] - 1, j2 = I.ng + I.N[1] - 1;
   const double* w = I.w[parity];
   const double* b = I.b[parity];
   double* w1 = I.w[parity ^ 1];
   double* b1 = I.b[parity ^ 1];
-  for (int t = threadIdx.x; t < T.wx * T.wy; t += blockDim.x) {
+  for (int t = tid; t < T.wx * T.wy; t += nthreads) {
     const int i = T.x0 + t % T.wx, j = T.y0 + t / T.wx;
     const long long c = (long long)j * I.nx + i;
 #pragma unroll
@@ -893,7 +893,7 @@ __global__ void __launch_bounds__(256, 2) k_corr2d(const Inst* __restrict__ inst
   const double dt = I.ds->dt;
   if (!(dt > 0.)) {
     // time has reached tmax: carry the state over unchanged
-    copy_tile(I, T, parity);
+    copy_tile(I, T, parity, threadIdx.x, blockDim.x);
     return;
   }
   // staged cells first, then the fluxes, EMFs and slopes
@@ -1127,7 +1127,7 @@ __global__ void __launch_bounds__(256, 2) k_corr2d_pq(const Inst* __restrict__ i
     const double dt = I.ds->dt;
     bool alive = true;
     if (!(dt > 0.)) {
-      copy_tile(I, T, parity);  // time has reached tmax: carry the state over (no staged data used)
+      copy_tile(I, T, parity, threadIdx.x, blockDim.x);  // time has reached tmax: carry the state over (no staged data used)
       // every thread has passed its parity-0 wait before phase 1 can complete
       __syncthreads();
     } else {

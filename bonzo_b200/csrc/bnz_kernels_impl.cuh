@@ -21,6 +21,7 @@ namespace BNZ_NS {
 #include "bnz_split_flux.cuh"
 #include "bnz_split.cuh"
 #include "bnz_fused.cuh"
+#include "bnz_walk2d.cuh"
 #include "bnz_fused3d.cuh"
 #include "bnz_split_tma.cuh"
 #include "bnz_adjoint_math.h"
@@ -258,16 +259,31 @@ inline int sm_count() {
 }
 
 namespace {
-// Blocks of 32 x 8 cells of the box, split::UPD_KZ z indices each.
-inline dim3 cell_grid(const plain::Box& b) {
-  const int kz = split::UPD_KZ;
+// Planes a block of k_ee, k_update or k_update_tma walks: 16, or on a grid of
+// few columns as many as leave the launch `want` blocks, at least 2.  A block
+// walks its planes one after the other, so a small grid wants shorter walks; a
+// walk's first plane costs loads that the next ones carry.  Measured, us for 6
+// or 8 steps of one grid alone (with three in flight), 16 planes throughout
+// against this: 97 x 65 x 50 2466 (1647) against 1930 (1639), 63^3 2976 (1782)
+// against 2074 (1782), 40^3 in the TMA form 1656 (757) against 976 (600); from
+// 128^3 up it is 16.
+inline int update_kz(const plain::Box& b, int want) {
+  const int cols = ((b.hi.x - b.lo.x + 32) / 32) * ((b.hi.y - b.lo.y + 8) / 8);
+  for (int kz = 16; kz > 2; kz /= 2)
+    if (cols * ((b.hi.z - b.lo.z + kz) / kz) >= want) return kz;
+  return 2;
+}
+
+// Blocks of 32 x 8 cells of the box, kz planes each.
+inline dim3 cell_grid(const plain::Box& b, int kz) {
   return dim3((b.hi.x - b.lo.x + 32) / 32, (b.hi.y - b.lo.y + 8) / 8, (b.hi.z - b.lo.z + kz) / kz);
 }
 
 // Walk length of a column walk: the faces a thread walks, so that the launch
 // holds about four times the blocks the device keeps resident (an even last
 // wave), at least `least` faces (a PLM walk starts with a slope that its
-// neighbour forms too: one in four at most) and at most 32.
+// neighbour forms too: one in four at most) and at most 32.  A grid of too few
+// faces to fill the device walks 2 or 1 instead.
 inline int walk_len(long long units, long long blocks_per_unit_row, int resident, int least) {
   const long long want = 4LL * resident;  // blocks
   long long parts = (want + blocks_per_unit_row - 1) / std::max(1LL, blocks_per_unit_row);
@@ -306,7 +322,8 @@ void launch_split_flux(const StepArgs& a, const double* w, const double* bf, con
     constexpr int sm = split::ColSmem<ORDER, CP>::BYTES;
     const int res = flux_resident(split::k_flux_march<AX, ORDER, RS, CP>, sm, per_sm);
     const long long nf = AX == 1 ? ny : nz, ncol = nx * (AX == 1 ? nz : ny), nbx = (ncol + NT - 1) / NT;
-    const int len = walk_len(nf, nbx, res, 4);
+    const long long faces = nf * ncol, room = (long long)res * NT;
+    const int len = walk_len(nf, nbx, res, faces < room / 4 ? 1 : faces < room ? 2 : 4);
     split::k_flux_march<AX, ORDER, RS, CP><<<dim3((unsigned)nbx, (unsigned)((nf + len - 1) / len)), NT, sm, a.stream>>>(
         a.g, w, bf, a.flx[AX], b, a.limiter, len, a.err);
   }
@@ -346,11 +363,13 @@ int split_stage(const StepArgs& a, const plain::Box& b, const double* w, double*
   if (g.dims >= 3) nl += split_flux<2>(a, order, w, bf, mkbox(il - 1, iu + 1, jl - 1, ju + 1, kl, ku + 1));
   {
     plain::Box be = mkbox(il, iu + 1, jl, g.dims >= 2 ? ju + 1 : 0, kl, g.dims >= 3 ? ku + 1 : 0);
-    split::k_ee<<<cell_grid(be), dim3(32, 8), 0, a.stream>>>(g, w, a.flx[0], a.flx[1], a.flx[2], a.ee, be);
+    const int kz = update_kz(be, 2 * sm_count());
+    split::k_ee<<<cell_grid(be, kz), dim3(32, 8), 0, a.stream>>>(g, w, a.flx[0], a.flx[1], a.flx[2], a.ee, be, kz);
   }
+  // (two blocks fit an SM without TMA, one with)
+  const int kz = update_kz(b, g.dims == 3 && a.smaps ? 60 : 200);
   if (g.dims == 3 && a.smaps) {
-    // the TMA-fed form (3D, even Ntot_x): blocks of 32 x 8 columns,
-    // split::UPD_KZ planes each
+    // the TMA-fed form (3D, even Ntot_x)
     constexpr size_t sm = sizeof(split::TmaSmem);
     static bool attr = false;  // once per floating-point build
     if (!attr) {
@@ -358,13 +377,12 @@ int split_stage(const StepArgs& a, const plain::Box& b, const double* w, double*
       attr = true;
     }
     const int b0map = b0 == a.bfld ? split::TM_BFLD : split::TM_BSAVE;
-    split::k_update_tma<<<cell_grid(b), dim3(32, 8), sm, a.stream>>>(g, w1, w, b1, bsave, a.smaps, b0map, b, dtp, fac,
-                                                                     a.src, a.grav[0], a.grav[1], a.grav[2], a.fdriv,
-                                                                     a.err);
+    split::k_update_tma<<<cell_grid(b, kz), dim3(32, 8), sm, a.stream>>>(
+        g, w1, w, b1, bsave, a.smaps, b0map, b, kz, dtp, fac, a.src, a.grav[0], a.grav[1], a.grav[2], a.fdriv, a.err);
     return nl + 2;
   }
-  split::k_update<<<cell_grid(b), dim3(32, 8), 0, a.stream>>>(
-      g, w1, a.prim, w, b1, b0, bsave, a.flx[0], a.flx[1], a.flx[2], a.ee, b, dtp, fac, a.src, a.grav[0],
+  split::k_update<<<cell_grid(b, kz), dim3(32, 8), 0, a.stream>>>(
+      g, w1, a.prim, w, b1, b0, bsave, a.flx[0], a.flx[1], a.flx[2], a.ee, b, kz, dtp, fac, a.src, a.grav[0],
       a.grav[1], a.grav[2], a.fdriv, a.err);
   return nl + 2;
 }
@@ -574,8 +592,36 @@ void launch_variant(const FusedLaunch& f, int parity) {
   if (f.events) cudaEventRecord(f.events[3], f.stream);
 }
 
+template <int ORDER, int RS, int LIM>
+void launch_walk(const FusedLaunch& f, const FusedTile* tiles, int nt, int parity) {
+  constexpr int sm = fused::WalkSmem<ORDER>::BYTES, nw = fused::WALK_NW;
+  static bool attrs = false;
+  if (!attrs) {
+    cudaFuncSetAttribute(fused::k_walk2d<ORDER, RS, LIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    cudaFuncSetAttribute(fused::k_walk2d<ORDER, RS, LIM>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    attrs = true;
+  }
+  if (nt < 1) return;
+  fused::k_walk2d<ORDER, RS, LIM><<<(nt + nw - 1) / nw, 32 * nw, sm, f.stream>>>(f.insts, tiles, nt, parity);
+}
+
+template <int RS>
+void launch_pred_corr_walk(const FusedLaunch& f, int parity) {
+  if (f.events) cudaEventRecord(f.events[1], f.stream);
+  launch_walk<0, RS, dev::LIM_VL>(f, f.tilesA, f.ntA, parity);
+  if (f.events) cudaEventRecord(f.events[2], f.stream);
+  if (f.limiter == dev::LIM_MC) launch_walk<1, RS, dev::LIM_MC>(f, f.tilesB, f.ntB, parity);
+  else if (f.limiter == dev::LIM_MM) launch_walk<1, RS, dev::LIM_MM>(f, f.tilesB, f.ntB, parity);
+  else launch_walk<1, RS, dev::LIM_VL>(f, f.tilesB, f.ntB, parity);
+  if (f.events) cudaEventRecord(f.events[3], f.stream);
+}
+
 template <int RS>
 void launch_pred_corr(const FusedLaunch& f, int parity) {
+  if (f.walk) {
+    launch_pred_corr_walk<RS>(f, parity);
+    return;
+  }
   // FUSED_VARIANTS in bnz_common.h; variants 1-7 are built for HLLD only
   if constexpr (RS != dev::RS_HLLD) {
     if (f.variant == 8) {

@@ -26,13 +26,11 @@
 
 namespace split {
 
-// k_ee and k_update: a thread walks UPD_KZ cells up z (blocks of 32 x 8
-// columns) and asks L2 for the inputs of the cell two planes ahead while it
+// k_ee and k_update: a thread walks kz cells up z (blocks of 32 x 8
+// columns; update_kz in bnz_kernels_impl.cuh) and asks L2 for the inputs of the cell two planes ahead while it
 // computes, since a cell's loads outnumber what its registers hold in flight.
 // (Staging each tile's inputs in shared memory by asynchronous copies first
 // measured slower: 2.3 and 0.66 ms per 256^3 launch against 1.8 and 0.47.)
-constexpr int UPD_KZ = 16;
-
 __device__ __forceinline__ void prefetch_l2(const double* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // ct.pyx:128-148: component COMP of the cell-centred EMF -(v x B) of cell c
@@ -48,12 +46,12 @@ __device__ __forceinline__ double ec_at(const double* __restrict__ w, long long 
 // stage input prim
 __global__ void k_ee(GridDev g, const double* __restrict__ w_in, const double* __restrict__ fx,
                      const double* __restrict__ fy, const double* __restrict__ fz, double* __restrict__ ee,
-                     plain::Box box) {
+                     plain::Box box, int kz) {
   const long long sv = g.sv, sy = g.nx, sz = (long long)g.nx * g.ny;
   const int i = box.lo.x + (int)(blockIdx.x * 32 + threadIdx.x);
   const int j = box.lo.y + (int)(blockIdx.y * 8 + threadIdx.y);
   if (i > box.hi.x || j > box.hi.y) return;
-  const int kb = box.lo.z + (int)blockIdx.z * UPD_KZ, ke = min(kb + UPD_KZ - 1, box.hi.z);
+  const int kb = box.lo.z + (int)blockIdx.z * kz, ke = min(kb + kz - 1, box.hi.z);
   for (int k = kb; k <= ke; ++k) {
     const long long c = plain::cidx(g, i, j, k);
     if (k + 2 <= ke) {
@@ -114,7 +112,7 @@ __global__ void __launch_bounds__(256, 2) k_update(GridDev g, double* w1, const 
                                                 const double* __restrict__ b0, double* __restrict__ bsave,
                                                 const double* __restrict__ fx, const double* __restrict__ fy,
                                                 const double* __restrict__ fz, const double* __restrict__ ee,
-                                                plain::Box box, const double* dtp, double fac, int src,
+                                                plain::Box box, int kz, const double* dtp, double fac, int src,
                                                 double gx, double gy, double gz, const double* __restrict__ fdriv,
                                                 unsigned* err) {
   const double dt = fac * *dtp;
@@ -128,7 +126,7 @@ __global__ void __launch_bounds__(256, 2) k_update(GridDev g, double* w1, const 
   const int i = box.lo.x + (int)(blockIdx.x * 32 + threadIdx.x);
   const int j = box.lo.y + (int)(blockIdx.y * 8 + threadIdx.y);
   if (i > box.hi.x || j > box.hi.y) return;
-  const int kb = box.lo.z + (int)blockIdx.z * UPD_KZ, ke = min(kb + UPD_KZ - 1, box.hi.z);
+  const int kb = box.lo.z + (int)blockIdx.z * kz, ke = min(kb + kz - 1, box.hi.z);
   const bool d2 = g.dims >= 2, d3 = g.dims >= 3;
   // the column's coordinates (loaded once: the stores below may alias them
   // for all the compiler knows)

@@ -56,7 +56,7 @@ __device__ __forceinline__ void issue_plane(TmaBuf& B, unsigned long long* bar, 
 __global__ void __launch_bounds__(256, 1) k_update_tma(GridDev g, double* w1, const double* __restrict__ w0,
                                                        double* __restrict__ b1, double* __restrict__ bsave,
                                                        const unsigned char* __restrict__ maps, int b0map,
-                                                       plain::Box box, const double* dtp, double fac, int src,
+                                                       plain::Box box, int kz, const double* dtp, double fac, int src,
                                                        double gx, double gy, double gz,
                                                        const double* __restrict__ fdriv, unsigned* err) {
   extern __shared__ __align__(128) unsigned char tma_smem[];
@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(256, 1) k_update_tma(GridDev g, double* w1, co
   const int x0 = (box.lo.x & ~1) + (int)blockIdx.x * 32, y0 = box.lo.y + (int)blockIdx.y * 8;
   const int i = x0 + tx, j = y0 + ty;
   const bool live = i <= box.hi.x && j <= box.hi.y;
-  const int kb = box.lo.z + (int)blockIdx.z * UPD_KZ, ke = min(kb + UPD_KZ - 1, box.hi.z);
+  const int kb = box.lo.z + (int)blockIdx.z * kz, ke = min(kb + kz - 1, box.hi.z);
   if (tid == 0) {
     fused::tma::bar_init(&S.bar[0], 1);
     fused::tma::bar_init(&S.bar[1], 1);

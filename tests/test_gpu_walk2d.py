@@ -1,0 +1,115 @@
+"""The strip walks of large 2D batches and grids (bnz_walk2d.cuh) and the tile
+shapes of small single grids.
+
+Both build from the same expressions as the tile kernels, so in the exact build
+the states must be equal bit for bit: a batch that walks against the same batch
+on the tile variant 9, a single grid against the split path, which shares no
+kernel with either.  Sizes put the strips' edges everywhere: one column or row
+more and less than a strip holds, grids of a few cells, both sides of the size
+where a batch or a grid starts to walk."""
+import numpy as np
+import pytest
+
+from bonzo_b200 import problems as P
+from bonzo_b200._lib import Batch, Context
+
+pytestmark = pytest.mark.gpu
+
+SMALL = [(4, 4), (5, 40), (33, 6), (29, 9), (30, 8), (31, 7), (60, 17), (61, 16), (59, 33), (90, 91), (121, 25)]
+LARGE = [(640, 640), (641, 600), (600, 641), (512, 640)]  # 1.5 M zones: the batch walks
+
+
+def _state(n, bc, seed):
+    gc = P.make_grid(n[0], n[1], 1, dims=2, bc=bc)
+    rng = np.random.default_rng(seed)
+    prim, bfld = np.zeros((9,) + gc.shape), np.zeros((3,) + gc.shape)
+    a = gc.active
+    shp = prim[0][a].shape
+    prim[0][a] = np.exp(0.2 * rng.standard_normal(shp))
+    for v in (1, 2, 3):
+        prim[v][a] = 0.3 * rng.standard_normal(shp)
+    prim[4][a] = np.exp(0.2 * rng.standard_normal(shp))
+    prim[5][a] = rng.random(shp)
+    for c, b in enumerate((0.5, -0.4, 0.3)):  # uniform: divergence free
+        bfld[c] = b
+    return prim, bfld
+
+
+BCS = [((0, 0), (0, 0), (0, 0)), ((1, 1), (2, 2), (0, 0)), ((2, 2), (0, 0), (0, 0)), ((0, 0), (1, 1), (0, 0))]
+
+
+@pytest.mark.parametrize("bc,kw", [(BCS[0], {}), (BCS[1], dict(limiter="mc")), (BCS[2], dict(rsolver="hll")),
+                                   (BCS[3], dict(rsolver="hllt", limiter="mm")),
+                                   (BCS[1], dict(grav=(0.1, -0.4, 0.0)))])
+def test_walking_batch_bitwise_vs_tiles(bc, kw):
+    grids = [dict(Nx=n[0], Ny=n[1], Nz=1, dims=2, bc=bc) for n in SMALL + LARGE]
+    walk = Batch(grids, exact_fp=True, cour=0.3, **kw)
+    tile = Batch(grids, exact_fp=True, cour=0.3, **kw)
+    tile.set_variant(9)
+    for q, n in enumerate(SMALL + LARGE):
+        s = _state(n, bc, q)
+        for b in (walk, tile):
+            b[q].set_state(*s)
+            b[q].init()
+    for b in (walk, tile):
+        b.advance(1e30, 3)
+    for q in range(len(grids)):
+        assert walk[q].time() == tile[q].time()
+        for x, y in zip(walk[q].get_state(), tile[q].get_state()):
+            assert np.array_equal(x, y), (q, grids[q])
+
+
+def test_walking_batch_stops_at_tmax():
+    """An instance at tmax is carried over unchanged while the others step."""
+    bc = BCS[0]
+    grids = [dict(Nx=n[0], Ny=n[1], Nz=1, dims=2, bc=bc) for n in SMALL + LARGE]
+    walk, tile = Batch(grids, exact_fp=True, cour=0.3), Batch(grids, exact_fp=True, cour=0.3)
+    tile.set_variant(9)
+    for q, n in enumerate(SMALL + LARGE):
+        s = _state(n, bc, q)
+        for b in (walk, tile):
+            b[q].set_state(*s)
+            b[q].init()
+    for b in (walk, tile):
+        b.advance(2e-3, 6)  # coarse grids arrive in one step, the large ones step on
+    steps = [walk[q].time()[1] for q in range(len(grids))]
+    assert min(steps) < max(steps)
+    for q in range(len(grids)):
+        assert walk[q].time() == tile[q].time()
+        for x, y in zip(walk[q].get_state(), tile[q].get_state()):
+            assert np.array_equal(x, y), q
+
+
+@pytest.mark.parametrize("n", [(4, 5), (13, 14), (14, 29), (64, 64), (201, 150), (256, 256), (270, 250), (499, 500),
+                               (500, 500), (501, 500), (640, 397)])
+@pytest.mark.parametrize("bc", BCS[:2])
+def test_single_grid_shapes_bitwise_vs_split(n, bc):
+    """14 x 14 tiles, 16 x 16 tiles and (from 250 000 cells) walks of one grid."""
+    s = _state(n, bc, n[0])
+    out = []
+    for path in ("fused", "split"):
+        c = Context(Nx=n[0], Ny=n[1], Nz=1, dims=2, bc=bc, exact_fp=True, cour=0.3, path=path)
+        c.set_state(*s)
+        c.init()
+        for _ in range(2):
+            c.step(0.2 / max(n) / 4)
+        out.append(c.get_state())
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("n", [(40, 40, 40), (41, 23, 37), (64, 30, 17), (97, 65, 50)])
+def test_short_update_walks_bitwise_vs_plain(n):
+    """3D grids of few columns: the update and EMF kernels walk fewer planes a block."""
+    bc = ((0, 0), (1, 1), (2, 2))
+    gc = P.make_grid(*n, dims=3, bc=bc)
+    prim, bfld = P.blast(gc, b_mag=0.4, b_angle=0.6, center=(0.45, 0.55, 0.5), radius=0.2, p_ratio=40.)
+    out = []
+    for path in ("plain", "split"):
+        c = Context(Nx=n[0], Ny=n[1], Nz=n[2], dims=3, bc=bc, exact_fp=True, cour=0.3, path=path)
+        c.set_state(prim, bfld)
+        c.init()
+        c.advance(1e30, max_steps=3)
+        out.append(c.get_state())
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
