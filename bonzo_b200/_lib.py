@@ -483,10 +483,9 @@ def riemann(rsolver, wl, wr, bx, gam, exact_fp=False):
     wl, wr = wl.contiguous(), wr.contiguous()
     bx = bx.contiguous() if bx is not None else None
     flux = torch.empty_like(wl)
-    err = torch.zeros(1, dtype=torch.int32, device=wl.device)
     rs = RS[rsolver] if isinstance(rsolver, str) else rsolver
     rc = L.bnz_riemann(rs, nvar, wl.data_ptr(), wr.data_ptr(), bx.data_ptr() if bx is not None else None,
-                       flux.data_ptr(), n, float(gam), int(bool(exact_fp)), err.data_ptr(),
+                       flux.data_ptr(), n, float(gam), int(bool(exact_fp)), None,
                        torch.cuda.current_stream().cuda_stream)
     if rc != BNZ_OK:
         raise BnzError(rc, "bnz_riemann failed")

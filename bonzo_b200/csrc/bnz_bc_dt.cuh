@@ -53,8 +53,9 @@ __global__ void k_bc_axis(GridDev g, int ax, double* prim, double* bfld, FieldLi
   const int a1 = ax == 0 ? g.i1 : ax == 1 ? g.j1 : g.k1;
   const int a2 = ax == 0 ? g.i2 : ax == 1 ? g.j2 : g.k2;
   const int o1 = ax == 0 ? 1 : 0, o2 = ax == 2 ? 1 : 2;  // the two other axes
-  const long long nother = (long long)N[o1] * N[o2];
-  const long long per_field = 2LL * ng * nother;
+  // (32-bit index arithmetic: fewer ghost cells than cells, plain::Box)
+  const unsigned nother = (unsigned)N[o1] * (unsigned)N[o2], n1 = N[o1];
+  const unsigned per_field = 2u * ng * nother;
   const int fi = blockIdx.y;
   if (fi >= fl.n) return;
   const int f = fl.f[fi];
@@ -65,13 +66,14 @@ __global__ void k_bc_axis(GridDev g, int ax, double* prim, double* bfld, FieldLi
   // along x the ghost layers of a row are neighbours in memory: the layer is
   // the fastest index there, so that a warp reads and writes a few rows'
   // ends instead of one double per row
-  const long long nl = 2LL * ng;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < per_field;
-       t += (long long)gridDim.x * blockDim.x) {
-    long long rest = ax == 0 ? t / nl : t % nother;
-    int layer = (int)(ax == 0 ? t % nl : t / nother);
-    int side = layer / ng, gl = layer % ng;
-    int c1 = (int)(rest % N[o1]), c2 = (int)(rest / N[o1]);
+  const unsigned nl = 2u * ng;
+  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < per_field; t += gridDim.x * blockDim.x) {
+    const unsigned h = ax == 0 ? t / nl : t / nother;
+    const unsigned rest = ax == 0 ? h : t - h * nother;
+    const int layer = (int)(ax == 0 ? t - h * nl : h);
+    const int side = layer >= ng ? 1 : 0, gl = layer - side * ng;
+    const unsigned hi = rest / n1;
+    const int c1 = (int)(rest - hi * n1), c2 = (int)hi;
     int d = side == 0 ? a1 - ng + gl : a2 + 1 + gl;
     int flag = side == 0 ? flag0 : flag1;
     int src;
@@ -85,18 +87,17 @@ __global__ void k_bc_axis(GridDev g, int ax, double* prim, double* bfld, FieldLi
   }
 }
 
-// new_dt.pyx:55-99 + 117: per-cell (|v_d| + c_f)/dx_d, max over active cells.
-// Non-negative doubles order like their bit patterns, so the global max is an
-// integer atomicMax on the bits.
+// new_dt.pyx:55-99 + 117: per-cell (|v_d| + c_f)/dx_d, max over active cells,
+// left in lane 0 of the block's first warp (true there).  32-bit index
+// arithmetic (plain::Box says why it suffices).
 // hydro: the hydro build's sound speed (no magnetic field).
-__global__ void k_cds_max(GridDev g, const double* __restrict__ w, unsigned long long* slot, int hydro) {
-  double m = 0.;
-  const int nxa = g.i2 - g.i1 + 1, nya = g.j2 - g.j1 + 1, nza = g.k2 - g.k1 + 1;
-  const long long n = (long long)nxa * nya * nza;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    int i = g.i1 + (int)(t % nxa);
-    long long r = t / nxa;
-    int j = g.j1 + (int)(r % nya), k = g.k1 + (int)(r / nya);
+__device__ __forceinline__ bool cds_block_max(const GridDev& g, const double* __restrict__ w, int hydro, double& m) {
+  m = 0.;
+  const unsigned nxa = g.i2 - g.i1 + 1, nya = g.j2 - g.j1 + 1, nza = g.k2 - g.k1 + 1;
+  const unsigned n = nxa * nya * nza;
+  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+    const unsigned r = t / nxa, q2 = r / nya;
+    const int i = g.i1 + (int)(t - r * nxa), j = g.j1 + (int)(r - q2 * nya), k = g.k1 + (int)q2;
     long long c = ((long long)k * g.ny + j) * g.nx + i;
     double ww[NM];
 #pragma unroll
@@ -113,22 +114,50 @@ __global__ void k_cds_max(GridDev g, const double* __restrict__ w, unsigned long
   int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (lane == 0) red[wid] = m;
   __syncthreads();
-  if (wid == 0) {
-    m = lane < (int)(blockDim.x >> 5) ? red[lane] : 0.;
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (lane == 0 && m > 0.) atomicMax(slot, (unsigned long long)__double_as_longlong(m));
-  }
+  if (wid != 0) return false;
+  m = lane < (int)(blockDim.x >> 5) ? red[lane] : 0.;
+  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  return lane == 0;
 }
 
-__global__ void k_dt_reset(DtState* ds) { ds->cdsmax_bits = 0ULL; }
-
 // new_dt.pyx:117 and vanleer.pyx:95-96: dt = cour/max, clipped to tmax.
-__global__ void k_dt_finalize(DtState* ds, double cour, int clip) {
-  double m = __longlong_as_double((long long)ds->cdsmax_bits);
-  double dt = cour / m;
+__device__ __forceinline__ void dt_of_max(DtState* ds, double mx, double cour, int clip) {
+  double dt = cour / mx;
   if (clip && ds->time + dt > ds->tmax) dt = ds->tmax - ds->time;
   if (clip && ds->time >= ds->tmax) dt = 0.;
   ds->dt = dt;
+}
+
+// The time step of a single grid in one launch.  Non-negative doubles order
+// like their bit patterns, so the global max is an integer atomicMax on the
+// bits.  A block adds its maximum and then itself to the count; the one that
+// completes the count reads the maximum, leaves both at zero for the next
+// launch and writes dt (no block waits for another).  Host-stepped grids are
+// bound by launches and the read-back: with this and no second launch to set an
+// unclipped dt, 10 steps of 201 x 150 took 695 us instead of 769.
+__global__ void k_cfl_dt(GridDev g, const double* __restrict__ w, DtState* ds, int hydro, double cour, int clip) {
+  double m;
+  if (!cds_block_max(g, w, hydro, m)) return;
+  if (m > 0.) atomicMax(&ds->cfl_bits, (unsigned long long)__double_as_longlong(m));
+  __threadfence();
+  if (atomicAdd(&ds->cfl_done, 1u) + 1u < gridDim.x) return;
+  __threadfence();
+  const double mx = __longlong_as_double((long long)atomicExch(&ds->cfl_bits, 0ULL));
+  ds->cfl_done = 0u;
+  dt_of_max(ds, mx, cour, clip);
+}
+
+// The same in three launches, for the instances of a split batch (whose launch
+// count reports them).
+__global__ void k_dt_reset(DtState* ds) { ds->cdsmax_bits = 0ULL; }
+
+__global__ void k_cds_max(GridDev g, const double* __restrict__ w, unsigned long long* slot, int hydro) {
+  double m;
+  if (cds_block_max(g, w, hydro, m) && m > 0.) atomicMax(slot, (unsigned long long)__double_as_longlong(m));
+}
+
+__global__ void k_dt_finalize(DtState* ds, double cour, int clip) {
+  dt_of_max(ds, __longlong_as_double((long long)ds->cdsmax_bits), cour, clip);
 }
 
 __global__ void k_dt_set(DtState* ds, double dt) { ds->dt = dt; }

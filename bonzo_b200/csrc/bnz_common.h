@@ -57,6 +57,8 @@ struct DtState {
   unsigned long long cdsmax_bits;  // max of (|v|+cf)/dx as a bit pattern
   long long step;
   unsigned long long cds_bits[2];  // fused path: CFL max of the state of parity p
+  unsigned long long cfl_bits;     // k_cfl_dt: the blocks' maximum so far, zero between launches
+  unsigned cfl_done;               // k_cfl_dt: blocks that have added theirs, zero between launches
 };
 
 // Fused 2D path: one grid ("instance") of a batch, as the kernels see it.

@@ -984,6 +984,7 @@ int bnz_advance(bnz_ctx* c, double tmax, int max_steps, double* time_out, long* 
   int n = 0;
   while (c->time < tmax && (max_steps <= 0 || n < max_steps)) {
     double dt;
+    bool on_device = false;  // the record's dt is the step's
     if (!c->md.fixdt) {
       StepArgs a = step_args(c);
       c->launches += c->L->new_dt(a, c->prim, c->d_ds, c->md.cour, 0);
@@ -991,11 +992,12 @@ int bnz_advance(bnz_ctx* c, double tmax, int max_steps, double* time_out, long* 
       CKC(cudaMemcpyAsync(&ds, c->d_ds, sizeof ds, cudaMemcpyDeviceToHost, c->stream));
       CKC(cudaStreamSynchronize(c->stream));
       dt = ds.dt;
-      if (c->time + dt > tmax) dt = tmax - c->time;
+      on_device = !(c->time + dt > tmax);
+      if (!on_device) dt = tmax - c->time;
     } else {
       dt = c->md.dt_fixed;
     }
-    c->launches += c->L->set_dt(c->stream, c->d_ds, dt);
+    if (!on_device) c->launches += c->L->set_dt(c->stream, c->d_ds, dt);
     int rc = step_impl(c, dt);
     if (rc) return rc;
     c->time += dt;
@@ -1748,7 +1750,7 @@ int batch_step_split(bnz_batch* b, bool host_dt) {
   const int n = (int)b->ctx.size();
   for (bnz_ctx* c : b->ctx) {
     StepArgs a = step_args(c);
-    if (!c->md.fixdt) c->launches += c->L->new_dt(a, c->prim, c->d_ds, c->md.cour, 1);
+    if (!c->md.fixdt) c->launches += c->L->new_dt_batch(a, c->prim, c->d_ds, c->md.cour);
     else c->launches += c->L->fixed_dt(c->stream, c->d_ds, c->md.dt_fixed);
   }
   std::vector<DtState> ds(host_dt ? n : 0);

@@ -455,9 +455,16 @@ int interp_bc_active(const StepArgs& a) {
 int new_dt(const StepArgs& a, const double* prim, DtState* ds, double cour, int clip) {
   const GridDev& g = a.g;
   long long n = (long long)(g.i2 - g.i1 + 1) * (g.j2 - g.j1 + 1) * (g.k2 - g.k1 + 1);
+  bcdt::k_cfl_dt<<<nblocks(n, 256, 148 * 8), 256, 0, a.stream>>>(g, prim, ds, a.hydro, cour, clip);
+  return 1;
+}
+
+int new_dt_batch(const StepArgs& a, const double* prim, DtState* ds, double cour) {
+  const GridDev& g = a.g;
+  long long n = (long long)(g.i2 - g.i1 + 1) * (g.j2 - g.j1 + 1) * (g.k2 - g.k1 + 1);
   bcdt::k_dt_reset<<<1, 1, 0, a.stream>>>(ds);
   bcdt::k_cds_max<<<nblocks(n, 256, 148 * 8), 256, 0, a.stream>>>(g, prim, &ds->cdsmax_bits, a.hydro);
-  bcdt::k_dt_finalize<<<1, 1, 0, a.stream>>>(ds, cour, clip);
+  bcdt::k_dt_finalize<<<1, 1, 0, a.stream>>>(ds, cour, 1);
   return 3;
 }
 

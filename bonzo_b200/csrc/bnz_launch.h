@@ -14,6 +14,7 @@ struct Launchers {
   int (*cons2prim_all)(const StepArgs&);
   int (*interp_bc_active)(const StepArgs&);
   int (*new_dt)(const StepArgs&, const double* prim, DtState* ds, double cour, int clip);
+  int (*new_dt_batch)(const StepArgs&, const double* prim, DtState* ds, double cour);
   int (*set_dt)(cudaStream_t, DtState*, double);
   int (*time_advance)(cudaStream_t, DtState*);
   int (*diff_dt_max)(const StepArgs&, const DiffArgs&, unsigned long long* slot);
@@ -41,6 +42,7 @@ struct Launchers {
   int cons2prim_all(const StepArgs&);                                                                \
   int interp_bc_active(const StepArgs&);                                                             \
   int new_dt(const StepArgs&, const double* prim, DtState* ds, double cour, int clip);              \
+  int new_dt_batch(const StepArgs&, const double* prim, DtState* ds, double cour);                  \
   int set_dt(cudaStream_t, DtState*, double);                                                        \
   int time_advance(cudaStream_t, DtState*);                                                          \
   int diff_dt_max(const StepArgs&, const DiffArgs&, unsigned long long* slot);                      \
@@ -65,7 +67,7 @@ BNZ_DECLARE_LAUNCHERS(fast)
   const Launchers NS::table = {NS::plain_predictor_corrector, NS::fused_step, NS::fused_time,       \
                                NS::fused_cds, NS::apply_bc,                                           \
                                NS::prim2cons_all, NS::cons2prim_all, NS::interp_bc_active,           \
-                               NS::new_dt, NS::set_dt, NS::time_advance, NS::diff_dt_max,            \
+                               NS::new_dt, NS::new_dt_batch, NS::set_dt, NS::time_advance, NS::diff_dt_max,            \
                                NS::diff_stage, NS::adj_step, NS::source,    \
                                NS::drive, NS::riemann_rows, NS::fused3_step, NS::fused3_time,        \
                                NS::fused3_cds, NS::split_predictor_corrector, NS::fixed_dt};
