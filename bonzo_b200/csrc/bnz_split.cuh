@@ -95,6 +95,23 @@ __global__ void k_ee(GridDev g, const double* __restrict__ w_in, const double* _
   }
 }
 
+// ct.pyx:15-91, the new z face of a 3D cell from the edge EMFs of its level,
+// ey at (i, i + 1) and ex at (j, j + 1).  k_update forms a face in two places,
+// at the first plane of a block's walk and as the upper face that the next
+// plane carries on.  The fast build rounds both alike (which products are
+// rounded before the differences is fixed here, as the carried form had it), so
+// that a result does not depend on where a walk starts (update_kz).
+__device__ __forceinline__ double z_face(double bz, double dtda, double dsx, double dsy, const double* ey,
+                                         const double* ex) {
+#if BNZ_FAST_MATH
+  const double dy = fma(dsy, ey[1], -__dmul_rn(dsy, ey[0])), dx = fma(-dsx, ex[0], __dmul_rn(dsx, ex[1]));
+  return fma(dtda, dx, fma(-dtda, dy, bz));
+#else
+  const double v = bz - dtda * (dsy * ey[1] - dsy * ey[0]);
+  return v + dtda * (dsx * ex[1] - dsx * ex[0]);
+#endif
+}
+
 // One stage's update of the cells of `box` (the stage's update range): the
 // plain path's k_advance_hydro, k_advance_b (the cell's lower faces, and its
 // upper ones on the range's last cells), k_interp_bc, k_source and
@@ -233,6 +250,7 @@ __global__ void __launch_bounds__(256, 2) k_update(GridDev g, double* w1, const 
     };
     auto bzf = [&](double bz, const double* ey, const double* ex) {
       const double dtda = dt / (dsx * dsy);
+      if (d3) return z_face(bz, dtda, dsx, dsy, ey, ex);
       double v = bz - dtda * (dsy * ey[1] - dsy * ey[0]);
       if (d2) v += dtda * (dsx * ex[1] - dsx * ex[0]);
       return v;
