@@ -37,14 +37,14 @@ BYTES_PER_ZONE = 192  # 9 conserved + 3 face-B doubles read once and written onc
 # b^(n+1) (3): 36 doubles per active zone.  The predictor reads 12 and writes
 # 12 per zone it covers (active zones plus two ghost rings).
 CORR_BYTES_PER_ZONE = 288
-# DRAM bytes per active zone of one corrector launch (dram__bytes_read.sum +
-# dram__bytes_write.sum), from an ncu capture of the persistent corrector on
-# the first 16 instances of this batch (scaled per zone).
-CORR_TRAFFIC_PER_ZONE = 269.9
-# FP64 flops per zone-update of the persistent kernels (2 x DFMA + DADD + DMUL
-# thread instructions, those of the division and square-root sequences
-# included), from the same capture: predictor 1196 + corrector 1343.
-FLOPS_PER_ZONE = 2539
+# Per kernel variant, from ncu captures on the first 16 instances of this batch
+# (scaled per zone): DRAM bytes per active zone of one corrector launch
+# (dram__bytes_read.sum + dram__bytes_write.sum), and FP64 flops per zone-update
+# of predictor and corrector (2 x DFMA + DADD + DMUL thread instructions, those
+# of the division and square-root sequences included).  Null for a variant that
+# was not captured.
+COUNTS = {8: dict(traffic=269.9, flops=1196 + 1343)}
+NO_COUNTS = dict(traffic=None, flops=None)
 
 
 def parse():
@@ -295,8 +295,8 @@ def run_ours(args, rank, world, dist):
     eng, ctxs, step, multi, count = make_engine(args.path, batch, stream)
     tune = None
     if args.path == "batch":
-        from bonzo_b200._lib import variant_label, variants
-        vs = variants()
+        from bonzo_b200._lib import WALK_VARIANT, variant_name, variants
+        vs = variants() + [(0, 0, 0, 0)]
         if args.variant is not None:
             # a fixed variant (profiling runs: the autotuner's choice under a profiler is not the real one)
             eng.set_variant(args.variant)
@@ -306,10 +306,11 @@ def run_ours(args, rank, world, dist):
             from bonzo_b200 import autotune
             best, ms = autotune.tune_batch(eng, [q["N"] for q, _, _, _ in batch], METHOD["rsolver"],
                                            METHOD["limiter"], steps=2, use_cache=False)
-        tune = {"chosen": {"tile": "%dx%d" % vs[best][:2], "staged_predictor": bool(vs[best][2]),
+        tune = {"chosen": {"variant": variant_name(best),
+                           "tile": "strips of one warp" if best == WALK_VARIANT else "%dx%d" % vs[best][:2],
+                           "staged_predictor": bool(vs[best][2]),
                            "persistent": ["none", "corrector", "predictor and corrector"][vs[best][3]]},
-                "ms_per_step": {variant_label(vs[v]): round(t, 4)
-                                for v, t in ms.items()}}
+                "ms_per_step": {variant_name(v): round(t, 4) for v, t in ms.items()}}
     for _ in range(args.warmup):
         step()
     if multi is not None:
@@ -367,12 +368,14 @@ def run_ours(args, rank, world, dist):
     # the step is FP64-issue bound: its FP64 rate against the measured FMA peak
     from bonzo_b200._lib import fp64_fma_peak
     fp64_peak = fp64_fma_peak()
-    fp64_achieved = FLOPS_PER_ZONE * zones / (ms_step * 1e-3) / 1e12
-    fp64 = {"achieved_tflops": round(fp64_achieved, 3), "peak_tflops": round(fp64_peak, 3),
-            "frac": round(fp64_achieved / fp64_peak, 4) if fp64_peak > 0 else None,
-            "flops_per_zone": FLOPS_PER_ZONE,
+    counts = COUNTS.get(best, NO_COUNTS) if tune else NO_COUNTS
+    fp64_achieved = None if counts["flops"] is None else counts["flops"] * zones / (ms_step * 1e-3) / 1e12
+    fp64 = {"achieved_tflops": None if fp64_achieved is None else round(fp64_achieved, 3),
+            "peak_tflops": round(fp64_peak, 3),
+            "frac": round(fp64_achieved / fp64_peak, 4) if fp64_achieved and fp64_peak > 0 else None,
+            "flops_per_zone": counts["flops"],
             "peak_source": "measured in this run (bnz_fp64_fma_peak: independent FMA chains on every SM)",
-            "flops_source": "ncu FP64 instruction counts of the persistent kernels on the first 16 instances"}
+            "flops_source": "ncu FP64 instruction counts of the kernels that ran, on the first 16 instances"}
     step_achieved = BYTES_PER_ZONE * zones / (ms_step * 1e-3) / 1e9
     step_roof = {"achieved": round(step_achieved, 1), "frac": round(step_achieved / peak, 4),
                  "bytes_per_zone": BYTES_PER_ZONE,
@@ -389,10 +392,12 @@ def run_ours(args, rank, world, dist):
         # achieved in the zone-update unit: 192 B per active zone per launch
         achieved = BYTES_PER_ZONE * zones / (kms["corrector"] * 1e-3) / 1e9
         own = CORR_BYTES_PER_ZONE * zones / (kms["corrector"] * 1e-3) / 1e9
-        traffic = None if CORR_TRAFFIC_PER_ZONE is None else int(CORR_TRAFFIC_PER_ZONE * zones)
+        traffic = None if counts["traffic"] is None else int(counts["traffic"] * zones)
         roofline = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                     "frac": round(achieved / peak, 4), "traffic": traffic, "peak_source": peak_src,
-                    "kernel": ("k_corr2d_pq (persistent corrector, one launch covers every instance)"
+                    "kernel": ("k_walk2d (corrector by strip walks, one launch covers every instance)"
+                               if tune and best == WALK_VARIANT else
+                               "k_corr2d_pq (persistent corrector, one launch covers every instance)"
                                if tune and vs[best][3] else
                                "k_corr2d (corrector, one launch covers every instance)"),
                     "bytes_per_zone": BYTES_PER_ZONE,

@@ -30,6 +30,7 @@ EXPORTS = [
     "bnz_batch_create", "bnz_batch_destroy", "bnz_batch_last_error", "bnz_batch_size",
     "bnz_batch_instance", "bnz_batch_advance", "bnz_batch_advance_timed", "bnz_batch_step_host", "bnz_batch_test_withhold_loads", "bnz_fp64_fma_peak", "bnz_fast_rcp", "bnz_batch_set_stream", "bnz_batch_launch_count",
     "bnz_batch_sync", "bnz_variant_count", "bnz_batch_set_variant", "bnz_batch_get_variant",
+    "bnz_batch_walk_variant", "bnz_get_variant",
     "bnz_batch_time_variant", "bnz_batch_autotune", "bnz_vl2_step_noalloc", "bnz_noalloc_last_error",
     "bnz_noalloc_check", "bnz_noalloc_scratch_bytes", "bnz_set_state_device", "bnz_get_state_device", "bnz_rollout_forward",
     "bnz_rollout_adjoint", "bnz_step_adjoint", "bnz_history", "bnz_div_b", "bnz_riemann", "bnz_snapshot", "bnz_snapshot_wait",
@@ -124,6 +125,8 @@ def load():
     L.bnz_variant_count.argtypes = [ip, ip, ip, ip, ip]
     L.bnz_batch_set_variant.argtypes = [vp, C.c_int]
     L.bnz_batch_get_variant.argtypes = [vp, ip]
+    L.bnz_batch_walk_variant.argtypes = [vp, ip]
+    L.bnz_get_variant.argtypes = [vp, ip]
     L.bnz_batch_time_variant.argtypes = [vp, C.c_int, C.c_int, _dp]
     L.bnz_batch_autotune.argtypes = [vp, C.c_int, ip, _dp]
     _lib = L
@@ -269,6 +272,14 @@ class Context:
         self._ck(self.L.bnz_advance(self.h, tmax, max_steps, C.byref(t), C.byref(s)))
         return t.value, s.value
 
+    @property
+    def variant(self):
+        """What a 2D grid on the fused path runs on, chosen by its size: a tile
+        variant's number or WALK_VARIANT (-1 elsewhere)."""
+        v = C.c_int()
+        self._ck(self.L.bnz_get_variant(self.h, C.byref(v)))
+        return v.value
+
     def last_nsts(self):
         n = C.c_int()
         self._ck(self.L.bnz_last_nsts(self.h, C.byref(n)))
@@ -371,6 +382,7 @@ class Batch:
         for q, gkw in enumerate(grids):
             arr[q] = grid_desc(**gkw)
         m = method_desc(**method)
+        self.charact_proj = bool(m.charact_proj)
         h = C.c_void_p()
         rc = self.L.bnz_batch_create(arr, n, C.byref(m), C.byref(h))
         self.h = h
@@ -453,6 +465,13 @@ class Batch:
     def set_variant(self, v):
         self._ck(self.L.bnz_batch_set_variant(self.h, int(v)))
 
+    @property
+    def walk_variant(self):
+        """WALK_VARIANT where this batch can take the strip walks, else None."""
+        v = C.c_int()
+        self._ck(self.L.bnz_batch_walk_variant(self.h, C.byref(v)))
+        return v.value if v.value >= 0 else None
+
     def time_variant(self, v, steps=2):
         """ms per batch step of variant v (state restored afterwards)."""
         ms = C.c_double()
@@ -515,7 +534,7 @@ def fast_rcp(x):
 
 
 def variants():
-    """[(tx, ty, staged, persistent)] of the fused kernel variants."""
+    """[(tx, ty, staged, persistent)] of the fused kernels' tile variants."""
     L = load()
     n = C.c_int()
     L.bnz_variant_count(C.byref(n), None, None, None, None)
@@ -528,3 +547,11 @@ def variant_label(v):
     """'15x14s' style name of a variant tuple: s = staged predictor, p = persistent
     corrector, pp = persistent predictor and corrector."""
     return "%dx%d%s%s" % (v[0], v[1], "s" if v[2] else "", "p" * v[3])
+
+
+WALK_VARIANT = 10  # the strip walks (BNZ_VARIANT_WALK), beyond the tile variants
+
+
+def variant_name(v):
+    """Name of a variant number: the label of its tiles, or 'walk'."""
+    return "walk" if v == WALK_VARIANT else variant_label(variants()[v])

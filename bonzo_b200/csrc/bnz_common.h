@@ -154,8 +154,8 @@ struct FusedTile {
 // Variants of the fused kernels the autotuner chooses from: tile shape
 // (cells along x, y), whether the predictor stages its input cells in shared
 // memory, and whether the stages run as persistent TMA-fed kernels.  A batch
-// starts on variant 8 (persistent, 15 x 14), a single grid on the shape that
-// grid_variant picks.
+// starts on variant 8 (persistent, 15 x 14) or, a large one, on the walks
+// (WALK_VARIANT), a single grid on what grid_variant picks.
 struct FusedVariant {
   int tx, ty, staged, persistent;
 };
@@ -179,19 +179,23 @@ inline bool fused_variant_built(int v, bool hlld) {
   return v == 0 || v == 8 || v == 9 || (hlld && v > 0 && v < FUSED_NVARIANT);
 }
 
-constexpr int BATCH_DEFAULT_VARIANT = 8;
+// Variant number of the strip walks (bnz_walk2d.cuh), which have no tile shape
+// of their own: strips of up to WALK_COLS columns and walk_rows rows, for every
+// Riemann solver and limiter, without characteristic slopes.
+constexpr int WALK_VARIANT = FUSED_NVARIANT, WALK_COLS = 30;
+// Tiles of a batch that does not walk.
+constexpr int BATCH_TILE_VARIANT = 8;
 
-// Strip walks (bnz_walk2d.cuh) instead of a variant's tiles, for a batch on its
-// default variant or a single grid, without characteristic slopes: from the
-// size where enough strips fill the device.  Measured, us a step, walks against
-// tiles: batches 0.94 M zones 441 / 423 (persistent tiles ahead), 3.2 M 1220 /
-// 1338, 4.8 M 1793 / 2018; single grids (whose tiles are not persistent) 384^2
-// 139 / 95, 512^2 146 / 151, 640^2 173 / 240, 1024^2 422 / 581.
+// Strip walks, without characteristic slopes: from the size where enough strips
+// fill the device.  Measured, us a step, walks against tiles: batches 0.94 M
+// zones 441 / 423 (persistent tiles ahead), 3.2 M 1220 / 1338, 4.8 M 1793 /
+// 2018; single grids (whose tiles are not persistent) 384^2 139 / 95, 512^2
+// 146 / 151, 640^2 173 / 240, 1024^2 422 / 581.
 constexpr long long WALK_MIN_BATCH = 1500000, WALK_MIN_GRID = 250000;
 // Rows of a strip: as many as leave every SM's 12 warps five strips each (a
 // strip forms its lowest row's faces besides its own), 8 to 32.
 inline int walk_rows(long long zones, int nsm) {
-  const long long r = zones / (30LL * 12 * 5 * nsm);
+  const long long r = zones / ((long long)WALK_COLS * 12 * 5 * nsm);
   return (int)(r < 8 ? 8 : r > 32 ? 32 : r);
 }
 // Tiles of a single grid below that size: the kernels end a phase in a barrier,
@@ -202,7 +206,8 @@ inline int walk_rows(long long zones, int nsm) {
 // against 142 / 397, 201 x 150 875 / 888 against 770 / 780 (host steps), 256^2
 // 288 / 474 against 308 / 576, 300^2 404 / 708 against 404 / 614, 384^2 647 /
 // 848 against 665 / 846.
-inline int grid_variant(int n0, int n1, int nsm) {
+inline int grid_variant(int n0, int n1, bool charact, int nsm) {
+  if ((long long)n0 * n1 >= WALK_MIN_GRID && !charact) return WALK_VARIANT;
   const int t14 = ((n0 + 13) / 14) * ((n1 + 13) / 14), t32 = ((n0 + 31) / 32) * ((n1 + 7) / 8);
   return t14 > 2 * nsm && t32 <= 2 * nsm ? 0 : 9;
 }
@@ -219,8 +224,7 @@ struct FusedLaunch {
   const FusedTile* tilesB;  // corrector tiles (active cells)
   int ntB;
   int rsolver, limiter, charact_proj;
-  int variant;
-  int walk;  // the tiles are strips of the walk kernels, whatever the variant
+  int variant;  // of FUSED_VARIANTS, or WALK_VARIANT (the tiles are strips)
   double cour;
   int dt_mode;
   double dt_fixed;

@@ -371,8 +371,10 @@ void make_strips(int inst, const int* lo, const int* n, int cols, int rows, std:
 void make_walk_strips(int inst, int N0, int N1, int ng, bool pred, int rows, std::vector<FusedTile>& out) {
   const int a = pred ? 1 : ng, g = pred ? 2 * ng - 2 : 0;
   const int lo[2] = {a, a}, n[2] = {N0 + g, N1 + g};
-  make_strips(inst, lo, n, 30, rows, out);
+  make_strips(inst, lo, n, WALK_COLS, rows, out);
 }
+
+static_assert(WALK_VARIANT == BNZ_VARIANT_WALK, "the walks' number in the C ABI");
 
 int device_sms() {
   int dev = 0, n = 0;
@@ -432,7 +434,6 @@ FusedLaunch fused_launch(const bnz_ctx* c, int dt_mode) {
   f.limiter = c->md.limiter;
   f.charact_proj = c->md.charact_proj;
   f.variant = c->variant;
-  f.walk = c->walk;
   f.cour = c->md.cour;
   f.dt_mode = dt_mode;
   f.dt_fixed = c->md.dt_fixed;
@@ -467,22 +468,21 @@ cudaError_t build_ctx3(bnz_ctx* c) {
   return e;
 }
 
-// (Re)build the single-grid tile lists for the context's variant.
+// The single-grid tile lists of the variant that grid_variant picks.
 cudaError_t build_ctx_tiles(bnz_ctx* c) {
-  const int n0 = c->i2 - c->i1 + 1, n1 = c->j2 - c->j1 + 1;
-  const long long zones = (long long)n0 * n1;
-  c->walk = zones >= WALK_MIN_GRID && !c->md.charact_proj;
-  c->variant = grid_variant(n0, n1, device_sms());
-  const FusedVariant& v = FUSED_VARIANTS[c->variant];
-  const int rows = walk_rows(zones, device_sms());
+  const int n0 = c->i2 - c->i1 + 1, n1 = c->j2 - c->j1 + 1, nsm = device_sms();
+  c->variant = grid_variant(n0, n1, c->md.charact_proj, nsm);
   std::vector<FusedTile> tiles;
-  if (c->walk) make_walk_strips(0, n0, n1, c->ng, true, rows, tiles);
-  else if (c->variant == 0) make_tiles(0, n0, n1, c->ng, true, v.tx, v.ty, tiles);
-  else make_tiles_uniform(0, n0, n1, c->ng, v.tx, v.ty, tiles);
-  c->ntA = (int)tiles.size();
-  if (c->walk) make_walk_strips(0, n0, n1, c->ng, false, rows, tiles);
-  else make_tiles(0, n0, n1, c->ng, false, v.tx, v.ty, tiles);
-  c->ntB = (int)tiles.size() - c->ntA;
+  for (int pred = 1; pred >= 0; --pred) {
+    if (c->variant == WALK_VARIANT) {
+      make_walk_strips(0, n0, n1, c->ng, pred, walk_rows((long long)n0 * n1, nsm), tiles);
+    } else {
+      const FusedVariant& v = FUSED_VARIANTS[c->variant];
+      if (pred && c->variant != 0) make_tiles_uniform(0, n0, n1, c->ng, v.tx, v.ty, tiles);
+      else make_tiles(0, n0, n1, c->ng, pred, v.tx, v.ty, tiles);
+    }
+    (pred ? c->ntA : c->ntB) = (int)tiles.size() - (pred ? 0 : c->ntA);
+  }
   if (c->d_tiles) cudaFree(c->d_tiles);
   c->d_tiles = nullptr;
   cudaError_t e = cudaMalloc((void**)&c->d_tiles, tiles.size() * sizeof(FusedTile));
@@ -1011,6 +1011,12 @@ int bnz_advance(bnz_ctx* c, double tmax, int max_steps, double* time_out, long* 
   return BNZ_OK;
 }
 
+int bnz_get_variant(const bnz_ctx* c, int* v) {
+  if (!c || !v) return BNZ_ERR_ARG;
+  *v = c->md.path == BNZ_PATH_FUSED && c->gd.dims == 2 ? c->variant : -1;
+  return BNZ_OK;
+}
+
 int bnz_last_nsts(const bnz_ctx* c, int* nsts) {
   if (!c || !nsts) return BNZ_ERR_ARG;
   *nsts = c->last_nsts;
@@ -1200,12 +1206,21 @@ int bnz_stream(bnz_ctx* c, void** s) {
 // four launches (per-instance dt, predictor tiles, corrector tiles, time).
 // ===========================================================================
 
+// A 2D batch's tiles (or strips) for one variant: the predictor's list, then
+// the corrector's, and where every instance starts in each (n + 1 entries).
+struct BatchTiles {
+  int variant = 0;
+  FusedTile* d = nullptr;
+  int ntA = 0, ntB = 0;
+  std::vector<int> offA, offB;
+};
+
 struct bnz_batch {
   std::vector<bnz_ctx*> ctx;
   bnz_method_desc md;
   FusedInst* d_inst = nullptr;
-  FusedTile* d_tiles = nullptr;
-  int ntA = 0, ntB = 0;
+  BatchTiles tiles;        // of the batch's variant
+  BatchTiles group_tiles;  // a walking batch's tiles of variant 8, once needed
   cudaStream_t stream = nullptr;
   bool own_stream = true;
   cudaGraphExec_t graph = nullptr;
@@ -1214,12 +1229,8 @@ struct bnz_batch {
   long long launches = 0;
   long long graph_launches = 0;
   double h_tmax = 0.;
-  int variant = 0;
-  bool walk = false;  // the tiles are strips of the walk kernels
   const Launchers* L = nullptr;
   std::string err;
-  // first predictor / corrector tile of every instance (n + 1 entries)
-  std::vector<int> offA, offB;
   // host-state stepping: copy-in and copy-out streams and their events
   cudaStream_t cin = nullptr, cout = nullptr;
   std::vector<cudaEvent_t> hev;
@@ -1267,32 +1278,44 @@ int bfail(bnz_batch* b, int code, const std::string& msg) {
       return bfail(b, BNZ_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(_e));        \
   } while (0)
 
-FusedLaunch batch_launch(const bnz_batch* b, int dt_mode) {
+// The tiles a step of the whole batch runs on (the test switch withholds TMA
+// loads, which the walks have none of: a walking batch then runs on tiles).
+const BatchTiles& step_tiles(const bnz_batch* b) {
+  return b->withhold && b->group_tiles.d ? b->group_tiles : b->tiles;
+}
+
+// One step of the instances q0 .. q1-1 on the tiles t.
+FusedLaunch batch_launch(const bnz_batch* b, int dt_mode, const BatchTiles& t, int q0, int q1) {
   FusedLaunch f;
   memset(&f, 0, sizeof f);
   f.insts = b->d_inst;
-  f.ninst = (int)b->ctx.size();
-  f.tilesA = b->d_tiles;
-  f.ntA = b->ntA;
-  f.tilesB = b->d_tiles + b->ntA;
-  f.ntB = b->ntB;
+  f.inst0 = q0;
+  f.ninst = q1 - q0;
+  f.tilesA = t.d + t.offA[q0];
+  f.ntA = t.offA[q1] - t.offA[q0];
+  f.tilesB = t.d + t.ntA + t.offB[q0];
+  f.ntB = t.offB[q1] - t.offB[q0];
   f.rsolver = b->md.rsolver;
   f.limiter = b->md.limiter;
   f.charact_proj = b->md.charact_proj;
-  f.variant = b->variant;
-  f.walk = b->walk;
+  f.variant = t.variant;
   f.cour = b->md.cour;
   f.dt_mode = dt_mode;
   f.dt_fixed = b->md.dt_fixed;
   f.err = b->ctx.empty() ? nullptr : b->ctx[0]->d_err;
   f.stream = b->stream;
-  if (FUSED_VARIANTS[b->variant].persistent && b->d_maps && !b->walk) {
+  const int persistent = t.variant == WALK_VARIANT ? 0 : FUSED_VARIANTS[t.variant].persistent;
+  if (persistent && b->d_maps) {
     f.wsmaps = b->d_maps;
     f.queue = b->d_queue;
     f.withhold = b->withhold;
-    if (FUSED_VARIANTS[b->variant].persistent == 2) f.wmaps = b->d_wmaps;
+    if (persistent == 2) f.wmaps = b->d_wmaps;
   }
   return f;
+}
+
+FusedLaunch batch_launch(const bnz_batch* b, int dt_mode) {
+  return batch_launch(b, dt_mode, step_tiles(b), 0, (int)b->ctx.size());
 }
 
 Fused3Launch batch_launch3(const bnz_batch* b, int dt_mode) {
@@ -1404,33 +1427,35 @@ bool ws_map3(const bnz_ctx* c, const double* base, void* map128) {
 
 namespace {
 
-// Tile lists of every instance for the batch's variant (predictor list first).
-int batch_build_tiles(bnz_batch* b) {
-  const FusedVariant& v = FUSED_VARIANTS[b->variant];
-  std::vector<FusedTile> tA, tB;
-  b->offA.assign(1, 0);
-  b->offB.assign(1, 0);
+// The total of the batch's zones.
+long long batch_zones(const bnz_batch* b) {
   long long zones = 0;
   for (const bnz_ctx* c : b->ctx) zones += (long long)(c->i2 - c->i1 + 1) * (c->j2 - c->j1 + 1);
-  // (the test switch withholds the tile kernels' TMA loads, so it keeps them)
-  b->walk = b->variant == BATCH_DEFAULT_VARIANT && !b->withhold && zones >= WALK_MIN_BATCH && !b->md.charact_proj;
-  const int rows = walk_rows(zones, device_sms());
+  return zones;
+}
+
+// Tile lists of every instance for a variant, and the tensor maps its kernels
+// read (one tile list of a batch has a persistent variant at most).
+int batch_build_tiles(bnz_batch* b, int variant, BatchTiles& t) {
+  const bool walk = variant == WALK_VARIANT;
+  const FusedVariant v = walk ? FusedVariant{0, 0, 0, 0} : FUSED_VARIANTS[variant];
+  std::vector<FusedTile> tA, tB;
+  t.variant = variant;
+  t.offA.assign(1, 0);
+  t.offB.assign(1, 0);
+  const int rows = walk_rows(batch_zones(b), device_sms());
   for (int q = 0; q < (int)b->ctx.size(); ++q) {
     const bnz_ctx* c = b->ctx[q];
-    if (b->walk) {
-      make_walk_strips(q, c->i2 - c->i1 + 1, c->j2 - c->j1 + 1, c->ng, true, rows, tA);
-      make_walk_strips(q, c->i2 - c->i1 + 1, c->j2 - c->j1 + 1, c->ng, false, rows, tB);
-      b->offA.push_back((int)tA.size());
-      b->offB.push_back((int)tB.size());
-      continue;
-    }
-    if (v.persistent == 2) make_tiles_uniform(q, c->i2 - c->i1 + 1, c->j2 - c->j1 + 1, c->ng, v.tx, v.ty, tA);
-    else make_tiles(q, c->i2 - c->i1 + 1, c->j2 - c->j1 + 1, c->ng, true, v.tx, v.ty, tA);
-    make_tiles(q, c->i2 - c->i1 + 1, c->j2 - c->j1 + 1, c->ng, false, v.tx, v.ty, tB);
-    b->offA.push_back((int)tA.size());
-    b->offB.push_back((int)tB.size());
+    const int n0 = c->i2 - c->i1 + 1, n1 = c->j2 - c->j1 + 1;
+    if (walk) make_walk_strips(q, n0, n1, c->ng, true, rows, tA);
+    else if (v.persistent == 2) make_tiles_uniform(q, n0, n1, c->ng, v.tx, v.ty, tA);
+    else make_tiles(q, n0, n1, c->ng, true, v.tx, v.ty, tA);
+    if (walk) make_walk_strips(q, n0, n1, c->ng, false, rows, tB);
+    else make_tiles(q, n0, n1, c->ng, false, v.tx, v.ty, tB);
+    t.offA.push_back((int)tA.size());
+    t.offB.push_back((int)tB.size());
   }
-  if (v.persistent && !b->walk) {
+  if (v.persistent) {
     static_assert(sizeof(CUtensorMap) == 128, "tensor maps are 128 bytes");
     // 6 maps per instance (TmaBox<tx, ty> in bnz_fused.cuh): ws with tx + 4
     // cells from an even column and ty + 4 rows; w[0], w[1] (9 fields) and
@@ -1450,13 +1475,13 @@ int batch_build_tiles(bnz_batch* b) {
               cell_map(c, c->wbuf[1], 9, cw, ch, &m[2]) && cell_map(c, c->bbuf[0], 3, cw, ch, &m[3]) &&
               cell_map(c, c->bbuf[1], 3, cw, ch, &m[4]) && cell_map(c, c->bfld_s, 2, pw, ph, &m[5]);
     }
-    for (FusedTile& t : tB) t.tma = ok[t.inst];
+    for (FusedTile& x : tB) x.tma = ok[x.inst];
     if (!b->d_maps) CKB(cudaMalloc((void**)&b->d_maps, maps.size() * sizeof(CUtensorMap)));
     if (!b->d_queue) CKB(cudaMalloc((void**)&b->d_queue, 2 * sizeof(unsigned)));
     CKB(cudaMemcpy(b->d_maps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice));
     CKB(cudaMemset(b->d_queue, 0, 2 * sizeof(unsigned)));
   }
-  if (v.persistent == 2 && !b->walk) {
+  if (v.persistent == 2) {
     // predictor: boxes of TmaBoxP<tx, ty> over w[0], w[1] (9 fields) and
     // b[0], b[1] (3 faces): tx + 2 cells from an even column, ty + 2 rows;
     // only full interior tiles use them
@@ -1469,28 +1494,43 @@ int batch_build_tiles(bnz_batch* b) {
       ok[q] = cell_map(c, c->wbuf[0], 9, bw, bh, &maps[4 * q]) && cell_map(c, c->wbuf[1], 9, bw, bh, &maps[4 * q + 1]) &&
               cell_map(c, c->bbuf[0], 3, bw, bh, &maps[4 * q + 2]) && cell_map(c, c->bbuf[1], 3, bw, bh, &maps[4 * q + 3]);
     }
-    for (FusedTile& t : tA) {
-      const bnz_ctx* c = b->ctx[t.inst];
+    for (FusedTile& x : tA) {
+      const bnz_ctx* c = b->ctx[x.inst];
       const int ng = c->ng, n0 = c->i2 - c->i1 + 1, n1 = c->j2 - c->j1 + 1;
-      const bool interior = t.x0 - 1 >= ng && t.x0 + t.wx <= ng + n0 - 1 && t.y0 - 1 >= ng &&
-                            t.y0 + t.wy <= ng + n1 - 1;
-      t.tma = !ok[t.inst] ? 0 : (interior && t.wx == v.tx && t.wy == v.ty) ? 1 : 2;
+      const bool interior = x.x0 - 1 >= ng && x.x0 + x.wx <= ng + n0 - 1 && x.y0 - 1 >= ng &&
+                            x.y0 + x.wy <= ng + n1 - 1;
+      x.tma = !ok[x.inst] ? 0 : (interior && x.wx == v.tx && x.wy == v.ty) ? 1 : 2;
     }
     if (!b->d_wmaps) CKB(cudaMalloc((void**)&b->d_wmaps, maps.size() * sizeof(CUtensorMap)));
     CKB(cudaMemcpy(b->d_wmaps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice));
   }
-  b->ntA = (int)tA.size();
-  b->ntB = (int)tB.size();
+  t.ntA = (int)tA.size();
+  t.ntB = (int)tB.size();
   tA.insert(tA.end(), tB.begin(), tB.end());
-  if (b->d_tiles) cudaFree(b->d_tiles);
-  b->d_tiles = nullptr;
-  CKB(cudaMalloc((void**)&b->d_tiles, tA.size() * sizeof(FusedTile)));
-  CKB(cudaMemcpy(b->d_tiles, tA.data(), tA.size() * sizeof(FusedTile), cudaMemcpyHostToDevice));
-  if (b->graph) {
-    cudaGraphExecDestroy(b->graph);
-    b->graph = nullptr;
-  }
+  if (t.d) cudaFree(t.d);
+  t.d = nullptr;
+  CKB(cudaMalloc((void**)&t.d, tA.size() * sizeof(FusedTile)));
+  CKB(cudaMemcpy(t.d, tA.data(), tA.size() * sizeof(FusedTile), cudaMemcpyHostToDevice));
   return BNZ_OK;
+}
+
+void drop_graph(bnz_batch* b) {
+  if (b->graph) cudaGraphExecDestroy(b->graph);
+  b->graph = nullptr;
+}
+
+// Makes v the batch's variant.
+int batch_use_variant(bnz_batch* b, int v) {
+  drop_graph(b);
+  if (b->group_tiles.d) cudaFree(b->group_tiles.d);
+  b->group_tiles.d = nullptr;
+  return batch_build_tiles(b, v, b->tiles);
+}
+
+// A walking batch's tiles with TMA loads (step_tiles).
+int batch_group_tiles(bnz_batch* b) {
+  if (b->tiles.variant != WALK_VARIANT || b->group_tiles.d) return BNZ_OK;
+  return batch_build_tiles(b, BATCH_TILE_VARIANT, b->group_tiles);
 }
 
 // Instance records, chunk lists and tensor maps of a 3D batch: every
@@ -1599,13 +1639,12 @@ int bnz_batch_create(const bnz_grid_desc* grids, int n, const bnz_method_desc* m
   b->L = b->ctx[0]->L;
   if (b->split) return BNZ_OK;
   if (b->dims3) {
-    b->variant = 0;
     return batch_build3(b);
   }
   CKB(cudaMalloc((void**)&b->d_inst, insts.size() * sizeof(FusedInst)));
   CKB(cudaMemcpy(b->d_inst, insts.data(), insts.size() * sizeof(FusedInst), cudaMemcpyHostToDevice));
-  b->variant = BATCH_DEFAULT_VARIANT;
-  return batch_build_tiles(b);
+  const bool walk = !md->charact_proj && batch_zones(b) >= WALK_MIN_BATCH;
+  return batch_use_variant(b, walk ? WALK_VARIANT : BATCH_TILE_VARIANT);
 }
 
 int bnz_batch_destroy(bnz_batch* b) {
@@ -1613,7 +1652,8 @@ int bnz_batch_destroy(bnz_batch* b) {
   if (b->stream) cudaStreamSynchronize(b->stream);
   for (bnz_ctx* c : b->ctx) bnz_destroy(c);
   if (b->d_inst) cudaFree(b->d_inst);
-  if (b->d_tiles) cudaFree(b->d_tiles);
+  if (b->tiles.d) cudaFree(b->tiles.d);
+  if (b->group_tiles.d) cudaFree(b->group_tiles.d);
   if (b->d_maps) cudaFree(b->d_maps);
   if (b->d_wmaps) cudaFree(b->d_wmaps);
   if (b->d_stage) cudaFree(b->d_stage);
@@ -2045,13 +2085,7 @@ int bnz_batch_step_host(bnz_batch* b, double* const* prim, double* const* bfld, 
   const int p0 = b->parity, p1 = (p0 + nsteps) & 1;
   for (int k = 0; k < nc; ++k) {
     const int q0 = cut[k], q1 = cut[k + 1];
-    FusedLaunch f = batch_launch(b, mode);
-    f.inst0 = q0;
-    f.ninst = q1 - q0;
-    f.tilesA = b->d_tiles + b->offA[q0];
-    f.ntA = b->offA[q1] - b->offA[q0];
-    f.tilesB = b->d_tiles + b->ntA + b->offB[q0];
-    f.ntB = b->offB[q1] - b->offB[q0];
+    const FusedLaunch f = batch_launch(b, mode, step_tiles(b), q0, q1);
     CKB(cudaStreamWaitEvent(b->stream, b->hev[2 + 2 * k], 0));
     if (staged) {
       // staging buffer -> the instances' buffers of the current parity
@@ -2104,14 +2138,9 @@ int bnz_batch_step_host(bnz_batch* b, double* const* prim, double* const* bfld, 
 int bnz_batch_test_withhold_loads(bnz_batch* b, int on) {
   if (!b) return BNZ_ERR_ARG;
   CKB(cudaStreamSynchronize(b->stream));
-  const int before = b->withhold;
   b->withhold = on ? 1 : 0;
-  if (!b->dims3 && before != b->withhold) return batch_build_tiles(b);  // (drops the graph)
-  if (b->graph) {  // a captured step holds the old value
-    cudaGraphExecDestroy(b->graph);
-    b->graph = nullptr;
-  }
-  return BNZ_OK;
+  drop_graph(b);  // a captured step holds the old value
+  return on && !b->dims3 ? batch_group_tiles(b) : BNZ_OK;
 }
 
 int bnz_batch_launch_count(const bnz_batch* b, long long* n) {
@@ -2142,18 +2171,25 @@ int bnz_variant_count(int* n, int* tx, int* ty, int* staged, int* persistent) {
 int bnz_batch_set_variant(bnz_batch* b, int v) {
   if (!b) return BNZ_ERR_ARG;
   if (b->dims3) return v == 0 ? BNZ_OK : bfail(b, BNZ_ERR_UNSUPPORTED, "3D batches have one kernel shape");
-  if (v < 0 || v >= FUSED_NVARIANT) return bfail(b, BNZ_ERR_ARG, "variant out of range");
-  if (!fused_variant_built(v, b->md.rsolver == BNZ_RS_HLLD))
+  if (v < 0 || (v >= FUSED_NVARIANT && v != WALK_VARIANT)) return bfail(b, BNZ_ERR_ARG, "variant out of range");
+  if (v == WALK_VARIANT && b->md.charact_proj)
+    return bfail(b, BNZ_ERR_UNSUPPORTED, "the walks have no characteristic slopes");
+  if (v != WALK_VARIANT && !fused_variant_built(v, b->md.rsolver == BNZ_RS_HLLD))
     return bfail(b, BNZ_ERR_UNSUPPORTED, "variants 1-7 are built for hlld only");
-  if (v == b->variant) return BNZ_OK;
+  if (v == b->tiles.variant) return BNZ_OK;
   CKB(cudaStreamSynchronize(b->stream));
-  b->variant = v;
-  return batch_build_tiles(b);
+  return batch_use_variant(b, v);
 }
 
 int bnz_batch_get_variant(const bnz_batch* b, int* v) {
   if (!b || !v) return BNZ_ERR_ARG;
-  *v = b->variant;
+  *v = b->tiles.variant;
+  return BNZ_OK;
+}
+
+int bnz_batch_walk_variant(const bnz_batch* b, int* v) {
+  if (!b || !v) return BNZ_ERR_ARG;
+  *v = b->dims3 || b->md.charact_proj ? -1 : WALK_VARIANT;
   return BNZ_OK;
 }
 
@@ -2162,7 +2198,7 @@ int bnz_batch_get_variant(const bnz_batch* b, int* v) {
 int bnz_batch_time_variant(bnz_batch* b, int v, int steps, double* ms) {
   if (!b || steps < 1) return BNZ_ERR_ARG;
   if (b->dims3) return bfail(b, BNZ_ERR_UNSUPPORTED, "3D batches have one kernel shape");
-  const int v0 = b->variant, p0 = b->parity;
+  const int v0 = b->tiles.variant, p0 = b->parity;
   int rc = bnz_batch_set_variant(b, v);
   if (rc) return rc;
   // save every instance's state of the current parity and its time record
@@ -2231,6 +2267,12 @@ int bnz_batch_autotune(bnz_batch* b, int steps, int* best, double* ms_per_varian
       }
     }
     if (ms_per_variant) ms_per_variant[v] = ms;
+  }
+  if (!b->md.charact_proj) {
+    double ms = -1.;
+    int rc = bnz_batch_time_variant(b, WALK_VARIANT, steps, &ms);
+    if (rc) return rc;
+    if (ms < best_ms) bv = WALK_VARIANT;
   }
   if (best) *best = bv;
   return bnz_batch_set_variant(b, bv);

@@ -51,7 +51,6 @@ struct bnz_ctx {
   unsigned char* d_smaps = nullptr;  // split path, 3D: the update kernel's tensor maps
   int graph_parity = -1;
   int variant = 0;
-  bool walk = false;  // fused 2D: the tiles are strips of the walk kernels
   // conduction scratch
   double* dscr = nullptr;
   DiffArgs da;

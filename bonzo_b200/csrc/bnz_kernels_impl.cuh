@@ -625,7 +625,7 @@ void launch_pred_corr_walk(const FusedLaunch& f, int parity) {
 
 template <int RS>
 void launch_pred_corr(const FusedLaunch& f, int parity) {
-  if (f.walk) {
+  if (f.variant == WALK_VARIANT) {
     launch_pred_corr_walk<RS>(f, parity);
     return;
   }

@@ -23,8 +23,8 @@
 
 namespace fused {
 
-constexpr int WALK_W = 30;
 constexpr int WALK_NW = 4;  // warps a block, one strip each
+static_assert(WALK_COLS + 2 == 32, "a lane a column of the strip, and one on either side");
 
 // a lane's slots between rows: [U] the x part of the row's flux differences,
 // then its hydro update, [BZ] likewise of bz; the row's x flux of by, its cell

@@ -215,15 +215,23 @@ int bnz_batch_test_withhold_loads(bnz_batch* batch, int on);
 int bnz_batch_launch_count(const bnz_batch* batch, long long* n);
 int bnz_batch_sync(bnz_batch* batch);
 
-/* Kernel variants (tile shape tx x ty, predictor staging, persistent
- * corrector fed by a tile queue with TMA-staged input) and the autotuner.
- * bnz_variant_count fills n and, if non-NULL, arrays of n entries.
- * bnz_batch_time_variant times `steps` steps of one variant on the live state
- * and restores the state afterwards; bnz_batch_autotune times every variant
- * and keeps the fastest (*best, and the per-variant ms, -1 where not built). */
+/* Kernel variants of 2D batches and the autotuner.  Variants 0 .. n-1 are tile
+ * shapes (tx x ty, predictor staging, persistent corrector fed by a tile queue
+ * with TMA-staged input); bnz_variant_count fills n and, if non-NULL, arrays of
+ * n entries.  BNZ_VARIANT_WALK is the strip walks, which have no tile shape and
+ * no characteristic slopes; a large batch starts on them, a smaller one on
+ * variant 8.  bnz_batch_walk_variant gives BNZ_VARIANT_WALK where the batch can
+ * take it, -1 where not.  bnz_batch_time_variant times `steps` steps of one
+ * variant on the live state and restores the state afterwards;
+ * bnz_batch_autotune times every variant and keeps the fastest (*best, and the
+ * ms of the n tile variants, -1 where not built).  bnz_get_variant tells what a
+ * single 2D grid on the fused path runs on, chosen by its size (-1 elsewhere). */
+#define BNZ_VARIANT_WALK 10
 int bnz_variant_count(int* n, int* tx, int* ty, int* staged, int* persistent);
 int bnz_batch_set_variant(bnz_batch* batch, int variant);
 int bnz_batch_get_variant(const bnz_batch* batch, int* variant);
+int bnz_batch_walk_variant(const bnz_batch* batch, int* variant);
+int bnz_get_variant(const bnz_ctx* ctx, int* variant);
 int bnz_batch_time_variant(bnz_batch* batch, int variant, int steps, double* ms);
 int bnz_batch_autotune(bnz_batch* batch, int steps, int* best, double* ms_per_variant);
 

@@ -61,6 +61,39 @@ def test_fastest_variant_kept_and_cached(cache):
     assert best2 == best and b2.chosen == best and b2.timed == [] and t2 == ms
 
 
+def test_cached_choice_is_for_the_same_kernels(cache):
+    """A choice timed without the strip walks (another batch, an older library)
+    does not answer for a batch that can walk, nor the reverse."""
+    nv = len(_lib.variants())
+    ms = _timings(nv)
+    autotune.tune_batch(FakeBatch(ms), [64] * 8)
+    b = FakeBatch({**ms, _lib.WALK_VARIANT: 0.1})
+    b.walk_variant = _lib.WALK_VARIANT
+    best, t = autotune.tune_batch(b, [64] * 8)
+    assert best == b.chosen == _lib.WALK_VARIANT and b.timed == list(range(nv)) + [_lib.WALK_VARIANT]
+    assert autotune.tune_batch(b, [64] * 8)[0] == _lib.WALK_VARIANT and len(b.timed) == nv + 1  # cached
+    b2 = FakeBatch(ms)
+    assert autotune.tune_batch(b2, [64] * 8)[0] == min(ms, key=ms.get) and len(b2.timed) == nv
+    d = json.loads(cache.read_text())
+    for e in d.values():
+        del e["variants"]
+    cache.write_text(json.dumps(d))
+    b3 = FakeBatch(ms)
+    autotune.tune_batch(b3, [64] * 8)
+    assert len(b3.timed) == nv
+
+
+def test_workload_key_tells_zones_and_slopes_apart():
+    even, uneven = [128] * 64, [16] * 48 + [464] * 16  # the same number of grids and mean side
+    assert autotune.workload_key(even, "hlld", "vl") != autotune.workload_key(uneven, "hlld", "vl")
+    assert autotune.workload_key(even, "hlld", "vl") != autotune.workload_key(even, "hlld", "vl", charact_proj=True)
+
+
+def test_variant_names():
+    names = [_lib.variant_name(v) for v in range(len(_lib.variants()) + 1)]
+    assert names[_lib.WALK_VARIANT] == "walk" and names[8] == "15x14pp" and len(set(names)) == len(names)
+
+
 def test_unsupported_variants_skipped(cache):
     nv = len(_lib.variants())
     ms = _timings(nv)

@@ -11,7 +11,7 @@ import numpy as np
 import pytest
 
 from bonzo_b200 import problems as P
-from bonzo_b200._lib import Batch, Context
+from bonzo_b200._lib import BNZ_ERR_UNSUPPORTED, WALK_VARIANT, Batch, BnzError, Context
 
 pytestmark = pytest.mark.gpu
 
@@ -45,6 +45,7 @@ def test_walking_batch_bitwise_vs_tiles(bc, kw):
     grids = [dict(Nx=n[0], Ny=n[1], Nz=1, dims=2, bc=bc) for n in SMALL + LARGE]
     walk = Batch(grids, exact_fp=True, cour=0.3, **kw)
     tile = Batch(grids, exact_fp=True, cour=0.3, **kw)
+    walk.set_variant(WALK_VARIANT)
     tile.set_variant(9)
     for q, n in enumerate(SMALL + LARGE):
         s = _state(n, bc, q)
@@ -64,6 +65,7 @@ def test_walking_batch_stops_at_tmax():
     bc = BCS[0]
     grids = [dict(Nx=n[0], Ny=n[1], Nz=1, dims=2, bc=bc) for n in SMALL + LARGE]
     walk, tile = Batch(grids, exact_fp=True, cour=0.3), Batch(grids, exact_fp=True, cour=0.3)
+    walk.set_variant(WALK_VARIANT)
     tile.set_variant(9)
     for q, n in enumerate(SMALL + LARGE):
         s = _state(n, bc, q)
@@ -78,6 +80,44 @@ def test_walking_batch_stops_at_tmax():
         assert walk[q].time() == tile[q].time()
         for x, y in zip(walk[q].get_state(), tile[q].get_state()):
             assert np.array_equal(x, y), q
+
+
+def test_variant_numbers_mean_one_kernel_each():
+    """A large batch starts on the walks; any tile variant can still be chosen
+    and is what runs, and a small batch can be made to walk."""
+    bc = BCS[0]
+    big = Batch([dict(Nx=n[0], Ny=n[1], Nz=1, dims=2, bc=bc) for n in LARGE], cour=0.3)
+    for q, n in enumerate(LARGE):
+        big[q].set_state(*_state(n, bc, q))
+        big[q].init()
+    assert big.variant == WALK_VARIANT
+    assert all(big.time_variant(v) > 0 for v in (8, WALK_VARIANT)) and big.variant == WALK_VARIANT
+    big.set_variant(8)
+    assert big.variant == 8
+    small = [dict(Nx=n[0], Ny=n[1], Nz=1, dims=2, bc=BCS[1]) for n in SMALL]
+    out = []
+    for v in (None, 8, 9, WALK_VARIANT):
+        b = Batch(small, exact_fp=True, cour=0.3)
+        assert b.variant == 8 and b.walk_variant == WALK_VARIANT
+        if v is not None:
+            b.set_variant(v)
+            assert b.variant == v
+        for q, n in enumerate(SMALL):
+            b[q].set_state(*_state(n, BCS[1], q))
+            b[q].init()
+        b.advance(1e30, 3)
+        out.append([c.get_state() for c in b.instances])
+    for o in out[1:]:
+        for s, s0 in zip(o, out[0]):
+            assert all(np.array_equal(x, y) for x, y in zip(s, s0))
+    for grids, kw in ((small, dict(charact_proj=1)), ([dict(Nx=8, Ny=8, Nz=8, dims=3, bc=bc)], {})):
+        b = Batch(grids, cour=0.3, **kw)
+        assert b.walk_variant is None
+        with pytest.raises(BnzError) as e:
+            b.set_variant(WALK_VARIANT)
+        assert e.value.code == BNZ_ERR_UNSUPPORTED
+    with pytest.raises(BnzError):
+        big.set_variant(WALK_VARIANT + 1)
 
 
 @pytest.mark.parametrize("n", [(4, 5), (13, 14), (14, 29), (64, 64), (201, 150), (256, 256), (270, 250), (499, 500),
