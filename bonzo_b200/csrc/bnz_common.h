@@ -183,7 +183,7 @@ inline bool fused_variant_built(int v, bool hlld) {
 // of their own: strips of up to WALK_COLS columns and walk_rows rows, for every
 // Riemann solver and limiter, without characteristic slopes.
 constexpr int WALK_VARIANT = FUSED_NVARIANT, WALK_COLS = 30;
-// Tiles of a batch that does not walk.
+// Tiles of a batch that does not walk, and of the parts of one that does.
 constexpr int BATCH_TILE_VARIANT = 8;
 
 // Strip walks, without characteristic slopes: from the size where enough strips

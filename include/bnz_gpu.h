@@ -198,6 +198,8 @@ int bnz_batch_advance_timed(bnz_batch* batch, double tmax, int nsteps, double* m
  * instances are split into nchunks groups of about equal size (0: 32) and
  * pipelined: the copy in of one group, the steps of the previous one and the
  * copy out of the one before that run at the same time on three streams.
+ * A batch on the strip walks takes variant 8's tiles for its groups (a part of
+ * the batch has too few strips), the walks only where it is one group.
  * Pinned host memory makes the copies asynchronous.  Returns when the copies
  * out are complete.  No counterpart in the reference, whose state lives in
  * host arrays between its steps (src/integration/vanleer.pyx:59-179). */

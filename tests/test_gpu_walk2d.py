@@ -153,3 +153,68 @@ def test_short_update_walks_bitwise_vs_plain(n):
         out.append(c.get_state())
     for x, y in zip(*out):
         assert np.array_equal(x, y)
+
+
+def _pinned(b):
+    import torch
+    host = []
+    for c in b.instances:
+        P_ = torch.empty((9,) + c.shape, dtype=torch.float64, pin_memory=True).numpy()
+        B_ = torch.empty((3,) + c.shape, dtype=torch.float64, pin_memory=True).numpy()
+        c.get_state_into(P_, None, B_)
+        host.append((P_, B_))
+    return [h[0] for h in host], [h[1] for h in host]
+
+
+@pytest.mark.parametrize("nchunks", [1, 2, 5, 0])
+def test_walking_batch_host_stepping(nchunks):
+    """Host stepping of a walking batch, as one group (walks) and in groups
+    (tiles), then walks on the device again: bitwise the batch on tiles."""
+    bc = BCS[1]
+    grids = [dict(Nx=n[0], Ny=n[1], Nz=1, dims=2, bc=bc) for n in SMALL + LARGE]
+    walk, tile = Batch(grids, exact_fp=True, cour=0.3), Batch(grids, exact_fp=True, cour=0.3)
+    walk.set_variant(WALK_VARIANT)
+    tile.set_variant(9)
+    for q, n in enumerate(SMALL + LARGE):
+        s = _state(n, bc, q)
+        for b in (walk, tile):
+            b[q].set_state(*s)
+            b[q].init()
+    P_, B_ = _pinned(walk)
+    walk.step_host(P_, B_, 1e30, 3, nchunks)
+    walk.advance(1e30, 2)
+    tile.advance(1e30, 3)
+    for q in range(len(grids)):
+        x = tile[q].get_state()
+        assert np.array_equal(P_[q], x[0]) and np.array_equal(B_[q], x[2]), q
+    tile.advance(1e30, 2)
+    assert walk.variant == WALK_VARIANT
+    for q in range(len(grids)):
+        assert walk[q].time() == tile[q].time()
+        for x, y in zip(walk[q].get_state(), tile[q].get_state()):
+            assert np.array_equal(x, y), q
+
+
+def test_walking_batch_host_stepping_is_not_slower_in_groups():
+    """The groups of a host-stepped batch are small: they must not take strips
+    cut for a launch of the whole batch (2.5 times the time of tiles)."""
+    import time
+    bc = BCS[0]
+    grids = [dict(Nx=320, Ny=320, Nz=1, dims=2, bc=bc)] * 32
+    ms = []
+    for v in (WALK_VARIANT, 8):
+        b = Batch(grids, cour=0.3)
+        assert b.variant == WALK_VARIANT
+        b.set_variant(v)
+        for q in range(len(grids)):
+            b[q].set_state(*_state((320, 320), bc, 0))
+            b[q].init()
+        P_, B_ = _pinned(b)
+        b.step_host(P_, B_, 1e30, 10)
+        best = 1e9
+        for _ in range(3):
+            t = time.perf_counter()
+            b.step_host(P_, B_, 1e30, 10)
+            best = min(best, time.perf_counter() - t)
+        ms.append(best)
+    assert ms[0] < 1.3 * ms[1], ms
