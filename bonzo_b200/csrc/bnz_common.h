@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include "../../include/bnz_gpu.h"
 
 // Grid geometry as the kernels see it.  Index conventions follow the
 // reference's GridCoord (src/coordinates/coord_c.h:19-99): Ntot cells per axis
@@ -186,11 +187,8 @@ constexpr int WALK_VARIANT = FUSED_NVARIANT, WALK_COLS = 30;
 // Tiles of a batch that does not walk, and of the parts of one that does.
 constexpr int BATCH_TILE_VARIANT = 8;
 
-// Strip walks, without characteristic slopes: from the size where enough strips
-// fill the device.  Measured, us a step, walks against tiles: batches 0.94 M
-// zones 441 / 423 (persistent tiles ahead), 3.2 M 1220 / 1338, 4.8 M 1793 /
-// 2018; single grids (whose tiles are not persistent) 384^2 139 / 95, 512^2
-// 146 / 151, 640^2 173 / 240, 1024^2 422 / 581.
+// Walks or tiles (no characteristic slopes in the walks): walks need enough
+// strips to fill the device, and strips that are not much narrower than a warp.
 constexpr long long WALK_MIN_BATCH = 1500000, WALK_MIN_GRID = 250000;
 // Rows of a strip: as many as leave every SM's 12 warps five strips each (a
 // strip forms its lowest row's faces besides its own), 8 to 32.
@@ -198,18 +196,51 @@ inline int walk_rows(long long zones, int nsm) {
   const long long r = zones / ((long long)WALK_COLS * 12 * 5 * nsm);
   return (int)(r < 8 ? 8 : r > 32 ? 32 : r);
 }
-// Tiles of a single grid below that size: the kernels end a phase in a barrier,
-// so a grid whose tiles fit one wave (two blocks an SM) wants tiles whose phases
-// take one round of the block's threads: 14 x 14.  Where those need a second
-// wave and 32 x 8 does not, 32 x 8.  Measured, us for 10 or 8 steps with three
-// grids in flight / of one grid alone, 32 x 8 against 14 x 14: 64^2 178 / 503
-// against 142 / 397, 201 x 150 875 / 888 against 770 / 780 (host steps), 256^2
-// 288 / 474 against 308 / 576, 300^2 404 / 708 against 404 / 614, 384^2 647 /
-// 848 against 665 / 846.
-inline int grid_variant(int n0, int n1, bool charact, int nsm) {
-  if ((long long)n0 * n1 >= WALK_MIN_GRID && !charact) return WALK_VARIANT;
-  const int t14 = ((n0 + 13) / 14) * ((n1 + 13) / 14), t32 = ((n0 + 31) / 32) * ((n1 + 7) / 8);
-  return t14 > 2 * nsm && t32 <= 2 * nsm ? 0 : 9;
+// Rows that the warps walk over n0 x n1 cells, a strip's two extra ones included.
+inline long long walk_steps(int n0, int n1, int rows) {
+  return (long long)((n0 + WALK_COLS - 1) / WALK_COLS) * (n1 + 2 * ((n1 + rows - 1) / rows));
+}
+inline long long tile_count(int n0, int n1, const FusedVariant& v) {
+  return (long long)((n0 + v.tx - 1) / v.tx) * ((n1 + v.ty - 1) / v.ty);
+}
+// A batch walks from WALK_MIN_BATCH zones, when `steps` rows of warps (both
+// stages) stand against enough of the `tiles` of variant 8.  Measured, time by
+// walks over time by tiles at steps / tiles: HLLD 7.6 0.87 (256^2 grids, 5 M
+// zones), 8.2 0.62 (31^2), 8.5 0.93, 8.9 0.99 (64^2, 5 M), 9.1 1.02 (128^2, 1.6
+// M) and 0.96 (40^2, 5 M), 9.3 0.67 (31^2, 1.6 M), 9.5 1.03 (64^2, 3 M), 10.0
+// 1.07, 11.2 1.10 (40 x 200); HLL 8.5 0.91, 9.1 1.00, 9.5 0.99 and 0.96, 10.0
+// 1.05; HLLT, whose walks cost most, 7.6 0.97, 8.0 0.92 (24^2), 8.1 1.04, 8.6
+// 1.12, 10.0 1.22.  Below 1.5 M zones the persistent tiles lead: at 0.94 M
+// zones of blasts 423 us a step against 441.
+inline bool batch_walks(int rsolver, long long zones, long long steps, long long tiles) {
+  const double most = rsolver == BNZ_RS_HLLD ? 9.4 : rsolver == BNZ_RS_HLLT ? 8. : 9.6;
+  return zones >= WALK_MIN_BATCH && steps <= most * tiles;
+}
+// What a single grid runs on.
+// Walks from WALK_MIN_GRID cells, us a step by walks / by 32 x 8 tiles of one
+// grid alone: HLLD 384^2 139 / 104, 500^2 130 / 154, 512^2 133 / 167, 1024^2 411
+// / 596, 80000 x 4 196 / 368; where strips are half empty and tiles full, tiles:
+// 31 x 10000 283 / 269 (20 steps a tile; the others up to 11).  HLLT 500^2 182 /
+// 166, 512^2 186 / 179, 576^2 204 / 225 (1296 tiles), so from 8 tiles an SM.
+// Tiles: the kernels end a phase in a barrier, and the phases of 14 x 14 tiles
+// are one round of a block's threads, those of 32 x 8 two.  Where 14 x 14 fit
+// one wave (two blocks an SM), or neither shape does and there are at most 1.4
+// times as many (1.75 on tall grids, whose 32 x 8 tiles are slower), 14 x 14;
+// us a step, 32 x 8 / 14 x 14, one grid alone (in brackets three in flight):
+// 64^2 52 / 36 (19 / 13), 224^2 58 / 40 (28 / 26), 256^2, 361 tiles against 256,
+// 58 / 64 (34 / 35), 288^2 88 / 67 (43 / 42), 384^2 104 / 95 (78 / 78), 4000 x
+// 60, 1.43 times, 149 / 153 (138 / 155), 60 x 4000 197 / 162 (173 / 154), 15000
+// x 20 with characteristic slopes, 1.52 times, 236 / 282.  Three grids of 2000 x
+// 16 at once pay for the one that gains alone: 54 / 39 (24 / 28).
+inline int grid_variant(int n0, int n1, int rsolver, bool charact, int nsm) {
+  const long long zones = (long long)n0 * n1;
+  const long long t14 = tile_count(n0, n1, FUSED_VARIANTS[9]), t32 = tile_count(n0, n1, FUSED_VARIANTS[0]);
+  if (zones >= WALK_MIN_GRID && !charact && walk_steps(n0, n1, walk_rows(zones, nsm)) <= 14 * t32 &&
+      (rsolver != BNZ_RS_HLLT || t32 >= 8LL * nsm))
+    return WALK_VARIANT;
+  if (t14 <= 2 * nsm) return 9;
+  if (t32 <= 2 * nsm) return 0;
+  return t14 <= (n1 > n0 ? 1.75 : 1.4) * t32 ? 9 : 0;
 }
 
 // dt modes of the fused step

@@ -471,7 +471,7 @@ cudaError_t build_ctx3(bnz_ctx* c) {
 // The single-grid tile lists of the variant that grid_variant picks.
 cudaError_t build_ctx_tiles(bnz_ctx* c) {
   const int n0 = c->i2 - c->i1 + 1, n1 = c->j2 - c->j1 + 1, nsm = device_sms();
-  c->variant = grid_variant(n0, n1, c->md.charact_proj, nsm);
+  c->variant = grid_variant(n0, n1, c->md.rsolver, c->md.charact_proj, nsm);
   std::vector<FusedTile> tiles;
   for (int pred = 1; pred >= 0; --pred) {
     if (c->variant == WALK_VARIANT) {
@@ -1647,7 +1647,18 @@ int bnz_batch_create(const bnz_grid_desc* grids, int n, const bnz_method_desc* m
   }
   CKB(cudaMalloc((void**)&b->d_inst, insts.size() * sizeof(FusedInst)));
   CKB(cudaMemcpy(b->d_inst, insts.data(), insts.size() * sizeof(FusedInst), cudaMemcpyHostToDevice));
-  const bool walk = !md->charact_proj && batch_zones(b) >= WALK_MIN_BATCH;
+  // a large batch walks where its strips cost less than its tiles would (both
+  // stages: the predictor covers two rings of ghost cells)
+  long long steps = 0, tiles = 0;
+  const int rows = walk_rows(batch_zones(b), device_sms());
+  for (const bnz_ctx* c : b->ctx) {
+    for (int ring = 0; ring <= 2; ring += 2) {
+      const int n0 = c->i2 - c->i1 + 1 + 2 * ring, n1 = c->j2 - c->j1 + 1 + 2 * ring;
+      steps += walk_steps(n0, n1, rows);
+      tiles += tile_count(n0, n1, FUSED_VARIANTS[BATCH_TILE_VARIANT]);
+    }
+  }
+  const bool walk = !md->charact_proj && batch_walks(md->rsolver, batch_zones(b), steps, tiles);
   return batch_use_variant(b, walk ? WALK_VARIANT : BATCH_TILE_VARIANT);
 }
 

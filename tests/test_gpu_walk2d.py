@@ -218,3 +218,25 @@ def test_walking_batch_host_stepping_is_not_slower_in_groups():
             best = min(best, time.perf_counter() - t)
         ms.append(best)
     assert ms[0] < 1.3 * ms[1], ms
+
+
+@pytest.mark.parametrize("grids,kw,variant", [
+    ([(640, 640)] * 4, {}, WALK_VARIANT), ([(640, 640)] * 4, dict(rsolver="hll"), WALK_VARIANT),
+    ([(640, 640)] * 4, dict(rsolver="hllt"), 8),          # its walks cost more than its tiles
+    ([(640, 640)] * 4, dict(charact_proj=1), 8),
+    ([(640, 640)] * 3, {}, 8),                            # too few zones
+    ([(25, 15000)] * 5, {}, WALK_VARIANT),                # one strip of 25 columns
+    ([(40, 9500)] * 4, {}, 8), ([(64, 6000)] * 4, dict(rsolver="hll"), 8)])  # half empty strips
+def test_batch_starts_on_the_faster_kernels(grids, kw, variant):
+    b = Batch([dict(Nx=n[0], Ny=n[1], Nz=1, dims=2) for n in grids], cour=0.3, **kw)
+    assert b.variant == variant
+
+
+@pytest.mark.parametrize("n,kw,variant", [
+    ((64, 64), {}, 9), ((224, 224), {}, 9), ((256, 256), {}, 0), ((384, 384), {}, 9), ((499, 500), {}, 9),
+    ((500, 500), {}, WALK_VARIANT), ((500, 500), dict(rsolver="hllt"), 9), ((500, 500), dict(charact_proj=1), 9),
+    ((640, 640), dict(rsolver="hllt"), WALK_VARIANT), ((4000, 60), {}, 0), ((60, 4000), {}, 9),
+    ((31, 10000), {}, 9), ((80000, 4), {}, WALK_VARIANT), ((80000, 4), dict(charact_proj=1), 0)])
+def test_single_grid_takes_the_faster_kernels(n, kw, variant):
+    assert Context(Nx=n[0], Ny=n[1], Nz=1, dims=2, path="fused", **kw).variant == variant
+    assert Context(Nx=n[0], Ny=n[1], Nz=1, dims=2, path="split", **kw).variant == -1
