@@ -279,17 +279,18 @@ inline dim3 cell_grid(const plain::Box& b, int kz) {
   return dim3((b.hi.x - b.lo.x + 32) / 32, (b.hi.y - b.lo.y + 8) / 8, (b.hi.z - b.lo.z + kz) / kz);
 }
 
-// Walk length of a column walk: the faces a thread walks, so that the launch
-// holds about four times the blocks the device keeps resident (an even last
-// wave), at least `least` faces (a PLM walk starts with a slope that its
-// neighbour forms too: one in four at most) and at most 32.  A grid of too few
-// faces to fill the device walks 2 or 1 instead.
-inline int walk_len(long long units, long long blocks_per_unit_row, int resident, int least) {
-  const long long want = 4LL * resident;  // blocks
-  long long parts = (want + blocks_per_unit_row - 1) / std::max(1LL, blocks_per_unit_row);
-  parts = std::max(parts, (units + 31) / 32);
-  parts = std::min(parts, std::max(1LL, units / least));
-  return (int)((units + parts - 1) / parts);
+// Faces a thread of a column walk takes: as few as put all walks on the device
+// at once, up to 16 (a second wave of a few blocks costs a whole walk); a larger
+// box takes about four waves of walks of at most 32 faces (an even last wave).
+// Measured, us a step of one grid, against four waves of at least four faces
+// with a column's walks in blocks of their own: 201 x 150 48 / 52 (HLLD, split
+// path), 30 x 3000 81 / 98, 512^2 with characteristic slopes 175 / 200, 32^3 75
+// / 83, 64^3 232 / 237; from 96^3 up the same.
+inline int walk_len(long long nf, long long ncol, long long room) {
+  for (int len = 1; len <= 16; ++len)
+    if (ncol * ((nf + len - 1) / len) <= room) return len;
+  const long long parts = std::max((4 * room + ncol - 1) / ncol, (nf + 31) / 32);
+  return (int)((nf + parts - 1) / parts);
 }
 
 // Resident blocks of a kernel on the whole device (asked for once per kernel).
@@ -321,11 +322,10 @@ void launch_split_flux(const StepArgs& a, const double* w, const double* bf, con
   } else {
     constexpr int sm = split::ColSmem<ORDER, CP>::BYTES;
     const int res = flux_resident(split::k_flux_march<AX, ORDER, RS, CP>, sm, per_sm);
-    const long long nf = AX == 1 ? ny : nz, ncol = nx * (AX == 1 ? nz : ny), nbx = (ncol + NT - 1) / NT;
-    const long long faces = nf * ncol, room = (long long)res * NT;
-    const int len = walk_len(nf, nbx, res, faces < room / 4 ? 1 : faces < room ? 2 : 4);
-    split::k_flux_march<AX, ORDER, RS, CP><<<dim3((unsigned)nbx, (unsigned)((nf + len - 1) / len)), NT, sm, a.stream>>>(
-        a.g, w, bf, a.flx[AX], b, a.limiter, len, a.err);
+    const long long nf = AX == 1 ? ny : nz, ncol = nx * (AX == 1 ? nz : ny);
+    const int len = walk_len(nf, ncol, (long long)res * NT), parts = (int)((nf + len - 1) / len);
+    split::k_flux_march<AX, ORDER, RS, CP><<<(unsigned)((ncol * parts + NT - 1) / NT), NT, sm, a.stream>>>(
+        a.g, w, bf, a.flx[AX], b, a.limiter, len, parts, a.err);
   }
 }
 

@@ -18,8 +18,10 @@
 // against 0.71 / 0.76 / 0.68 for one thread per face reading global memory.
 // Instructions per PLM face fell from 1240 to 770 (no tile coordinates, one
 // slope per face), issue rose from 43 to 47 % of the slots; 16 (PLM march) to
-// 20 warps an SM, the most whose registers do not spill (a spill costs more
-// than the warps it buys: PLM march at 20 warps and 96 registers 0.80).
+// 20 warps an SM (a spill costs more than the warps it buys there: PLM march at
+// 20 warps and 96 registers 0.80).  Characteristic slopes run at 16 warps and
+// 128 registers: one 512^2 grid 175 us a step at 12 warps, 169 at 16; 128^3 1521
+// and 1471.
 // Included inside the per-floating-point-mode namespace, after bnz_plain.cuh.
 #pragma once
 
@@ -144,21 +146,24 @@ __device__ __forceinline__ void col_slopes_rt(int lim, const double* m, const do
 // on its right), in the global variable order (the normal field entry, which
 // nothing reads, is not stored).  ORDER 0: donor cell (reconstr_c.c:8-22);
 // ORDER 1: PLM with limiter lim (reconstr_c.c:29-91), in characteristic
-// variables with CP.  Normal field from the face array bf.  Block x: 128
-// columns of the (x, other axis) plane of the box; block y: `len` faces.
+// variables with CP.  Normal field from the face array bf.  The columns of the
+// (x, other axis) plane of the box are cut into `parts` walks of `len` faces;
+// the threads take the walks of all columns part by part, so that a plane of
+// few columns still fills its blocks.
 template <int AX, int ORDER, int RS, int CP>
-__global__ void __launch_bounds__(FLUX_NT, CP ? 3 : ORDER ? 4 : 5)
+__global__ void __launch_bounds__(FLUX_NT, ORDER ? 4 : 5)
     k_flux_march(GridDev g, const double* __restrict__ w, const double* __restrict__ bf, double* __restrict__ F,
-                 plain::Box box, int lim, int len, unsigned* err) {
+                 plain::Box box, int lim, int len, int parts, unsigned* err) {
   using V = RowVars<CP>;
   constexpr int ST = FLUX_NT, RS_ = V::NV * ST;  // stride between a thread's values, between its rows
   constexpr int OAX = AX == 1 ? 2 : 1;
   extern __shared__ __align__(16) double flux_smem[];
   const int nxb = box.hi.x - box.lo.x + 1, no = ax_of(box.hi, OAX) - ax_of(box.lo, OAX) + 1;
-  const int col = blockIdx.x * ST + threadIdx.x;
-  if (col >= nxb * no) return;
+  const unsigned t = blockIdx.x * ST + threadIdx.x, ncol = (unsigned)nxb * no;
+  const int part = (int)(t / ncol), col = (int)(t - part * ncol);
+  if (part >= parts) return;
   const int i = box.lo.x + col % nxb, o = ax_of(box.lo, OAX) + col / nxb;
-  const int a0 = ax_of(box.lo, AX) + (int)blockIdx.y * len, a1 = min(a0 + len - 1, ax_of(box.hi, AX));
+  const int a0 = ax_of(box.lo, AX) + part * len, a1 = min(a0 + len - 1, ax_of(box.hi, AX));
   const long long sv = g.sv, sy = g.nx, sz = (long long)g.nx * g.ny;
   const long long sa = AX == 1 ? sy : sz, so = AX == 1 ? sz : sy;
   const long long c0 = i + o * so;
@@ -188,10 +193,10 @@ __global__ void __launch_bounds__(FLUX_NT, CP ? 3 : ORDER ? 4 : 5)
     col_slopes_rt<CP, ST, ST>(lim, r0, r1, r2, d, l, true, g.gam);
     row(r0, a0 + 1);
     cpa::commit();
-    double* t = r0;
+    double* q = r0;
     r0 = r1;
     r1 = r2;
-    r2 = t;
+    r2 = q;
   } else {
     row(r0, a0 - 1);
     row(r1, a0);
@@ -217,10 +222,10 @@ __global__ void __launch_bounds__(FLUX_NT, CP ? 3 : ORDER ? 4 : 5)
       if (n != BX) Fc[plain::perm<AX>(n) * sv] = fl[n];
     if (!ORDER && f + 2 <= a1) row(r0, f + 2);
     cpa::commit();
-    double* t = r0;
+    double* q = r0;
     r0 = r1;
     r1 = r2;
-    r2 = t;
+    r2 = q;
   }
   if (e) atomicOr(err, e);
 }
@@ -256,7 +261,7 @@ struct RowSmem {
 // the face on its left (the next segment starts at this one's last entry), so
 // 31 faces a segment; with donor cells all 32.  Warp q walks `len` segments.
 template <int ORDER, int RS, int CP>
-__global__ void __launch_bounds__(FLUX_NT, CP ? 3 : 5)
+__global__ void __launch_bounds__(FLUX_NT, CP ? 4 : 5)
     k_flux_row(GridDev g, const double* __restrict__ w, const double* __restrict__ bf, double* __restrict__ F,
                plain::Box box, int lim, int len, unsigned* err) {
   using V = RowVars<CP>;

@@ -13,6 +13,9 @@ pytestmark = pytest.mark.gpu
 
 SIZES = [(4, 4, 4), (5, 7, 4), (28, 5, 4), (29, 4, 6), (30, 6, 5), (31, 5, 5), (32, 4, 4), (33, 5, 4), (59, 4, 5),
          (60, 5, 4), (61, 4, 4), (4, 40, 5), (5, 4, 41), (6, 33, 1), (64, 4, 1), (27, 70, 1), (200, 1, 1), (25, 1, 1)]
+# columns whose walks share blocks: one walk a column and several, a block of one
+# walk of many columns, lanes of a warp in two walks
+SIZES += [(30, 600, 1), (3, 900, 1), (125, 33, 1), (126, 130, 1), (400, 300, 1), (40, 41, 42)]
 
 
 def _state(n, reconstr, hydro, seed):
