@@ -10,6 +10,7 @@
 
 #include "bnz_common.h"
 #include "bnz_launch.h"
+#include "bnz_per_device.h"
 
 namespace BNZ_NS {
 
@@ -248,14 +249,42 @@ int plain_predictor_corrector(const StepArgs& a, const double* dtp) {
   return nl + 2;
 }
 
-// SM count of the current device (cached per device).
+// (-1 where it cannot be told)
+inline int current_device() {
+  int dev = -1;
+  return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;
+}
+
+// SM count of the current device.
 inline int sm_count() {
-  static int nsm[64] = {0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) dev = 0;
-  if (!nsm[dev]) cudaDeviceGetAttribute(&nsm[dev], cudaDevAttrMultiProcessorCount, dev);
-  return std::max(1, nsm[dev]);
+  static PerDevice nsm;
+  return nsm.get(current_device(), [] {
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return std::max(1, n);
+  });
+}
+
+// Resident blocks of a kernel on an SM, after `set` has set its attributes.
+template <class K, class F>
+int resident(PerDevice& once, K kernel, int threads, size_t smem, F set) {
+  return once.get(current_device(), [&] {
+    set();
+    int n = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem);
+    return std::max(1, n);
+  });
+}
+
+// Allows a kernel `smem` bytes of dynamic shared memory.
+template <class K>
+void allow_smem(PerDevice& once, K kernel, size_t smem, bool all_shared = false) {
+  once.get(current_device(), [&] {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (all_shared) cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    return 1;
+  });
 }
 
 namespace {
@@ -293,21 +322,17 @@ inline int walk_len(long long nf, long long ncol, long long room) {
   return (int)((nf + parts - 1) / parts);
 }
 
-// Resident blocks of a kernel on the whole device (asked for once per kernel).
+// Resident blocks of a flux kernel on the whole device.
 template <class K>
-int flux_resident(K kernel, int smem, int& cache) {
-  if (!cache) {
+int flux_resident(K kernel, int smem, PerDevice& once) {
+  return sm_count() * resident(once, kernel, split::FLUX_NT, smem, [&] {
     cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, split::FLUX_NT, smem);
-    cache = std::max(1, n);
-  }
-  return cache * sm_count();
+  });
 }
 
 template <int AX, int ORDER, int RS, int CP>
 void launch_split_flux(const StepArgs& a, const double* w, const double* bf, const plain::Box& b) {
-  static int per_sm = 0;
+  static PerDevice per_sm;
   const long long nx = b.hi.x - b.lo.x + 1, ny = b.hi.y - b.lo.y + 1, nz = b.hi.z - b.lo.z + 1;
   constexpr int NT = split::FLUX_NT;
   if constexpr (AX == 0) {
@@ -371,11 +396,8 @@ int split_stage(const StepArgs& a, const plain::Box& b, const double* w, double*
   if (g.dims == 3 && a.smaps) {
     // the TMA-fed form (3D, even Ntot_x)
     constexpr size_t sm = sizeof(split::TmaSmem);
-    static bool attr = false;  // once per floating-point build
-    if (!attr) {
-      cudaFuncSetAttribute(split::k_update_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-      attr = true;
-    }
+    static PerDevice attr;  // (per floating-point build)
+    allow_smem(attr, split::k_update_tma, sm);
     const int b0map = b0 == a.bfld ? split::TM_BFLD : split::TM_BSAVE;
     split::k_update_tma<<<cell_grid(b, kz), dim3(32, 8), sm, a.stream>>>(
         g, w1, w, b1, bsave, a.smaps, b0map, b, kz, dtp, fac, a.src, a.grav[0], a.grav[1], a.grav[2], a.fdriv, a.err);
@@ -521,11 +543,8 @@ namespace {
 template <int TX, int TY, int RS, int LIM>
 void launch_corr(const FusedLaunch& f, int parity) {
   constexpr size_t smB = fused::Smem<TX, TY, 2>::bytes;
-  static bool attrs = false;
-  if (!attrs) {
-    cudaFuncSetAttribute(fused::k_corr2d<TX, TY, RS, LIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smB);
-    attrs = true;
-  }
+  static PerDevice attrs;
+  allow_smem(attrs, fused::k_corr2d<TX, TY, RS, LIM>, smB);
   fused::k_corr2d<TX, TY, RS, LIM><<<f.ntB, 256, smB, f.stream>>>(f.insts, f.tilesB, parity, f.charact_proj);
 }
 
@@ -533,12 +552,10 @@ void launch_corr(const FusedLaunch& f, int parity) {
 template <int TX, int TY, int RS, int LIM>
 void launch_corr_pq(const FusedLaunch& f, int parity) {
   constexpr size_t sm = fused::TmaBox<TX, TY>::smem_bytes;
-  static int per_sm = 0;
-  if (!per_sm) {
+  static PerDevice once;
+  const int per_sm = resident(once, fused::k_corr2d_pq<TX, TY, RS, LIM>, 256, sm, [&] {
     cudaFuncSetAttribute(fused::k_corr2d_pq<TX, TY, RS, LIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fused::k_corr2d_pq<TX, TY, RS, LIM>, 256, sm);
-    if (per_sm < 1) per_sm = 1;
-  }
+  });
   const int grid = std::min(f.ntB, per_sm * sm_count());
   if (grid < 1) return;
   fused::k_corr2d_pq<TX, TY, RS, LIM><<<grid, 256, sm, f.stream>>>(f.insts, f.tilesB, f.ntB, parity,
@@ -548,12 +565,10 @@ void launch_corr_pq(const FusedLaunch& f, int parity) {
 template <int TX, int TY, int RS>
 void launch_pred_pq(const FusedLaunch& f, int parity) {
   constexpr size_t sm = fused::TmaBoxP<TX, TY>::smem_bytes;
-  static int per_sm = 0;
-  if (!per_sm) {
+  static PerDevice once;
+  const int per_sm = resident(once, fused::k_pred2d_pq<TX, TY, RS>, 256, sm, [&] {
     cudaFuncSetAttribute(fused::k_pred2d_pq<TX, TY, RS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fused::k_pred2d_pq<TX, TY, RS>, 256, sm);
-    if (per_sm < 1) per_sm = 1;
-  }
+  });
   const int grid = std::min(f.ntA, per_sm * sm_count());
   if (grid < 1) return;
   fused::k_pred2d_pq<TX, TY, RS><<<grid, 256, sm, f.stream>>>(f.insts, f.tilesA, f.ntA, parity, f.wmaps,
@@ -575,12 +590,8 @@ template <int TX, int TY, int RS, int STAGED>
 void launch_variant(const FusedLaunch& f, int parity) {
   constexpr int TXA = TX + 4, TYA = TY + 4;  // predictor tiles grow by the ghost rings
   constexpr size_t smA = fused::Smem<TXA, TYA, STAGED ? 1 : 0>::bytes;
-  static bool attrs = false;
-  if (!attrs) {
-    cudaFuncSetAttribute(fused::k_pred2d<TXA, TYA, RS, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smA);
-    attrs = true;
-  }
+  static PerDevice attrs;
+  allow_smem(attrs, fused::k_pred2d<TXA, TYA, RS, STAGED>, smA);
   if (f.events) cudaEventRecord(f.events[1], f.stream);
   bool done = false;
   if constexpr (((TX == 15 && TY == 14) || (TX == 14 && TY == 14)) && STAGED == 0) {
@@ -602,12 +613,8 @@ void launch_variant(const FusedLaunch& f, int parity) {
 template <int ORDER, int RS, int LIM>
 void launch_walk(const FusedLaunch& f, const FusedTile* tiles, int nt, int parity) {
   constexpr int sm = fused::WalkSmem<ORDER>::BYTES, nw = fused::WALK_NW;
-  static bool attrs = false;
-  if (!attrs) {
-    cudaFuncSetAttribute(fused::k_walk2d<ORDER, RS, LIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    cudaFuncSetAttribute(fused::k_walk2d<ORDER, RS, LIM>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    attrs = true;
-  }
+  static PerDevice attrs;
+  allow_smem(attrs, fused::k_walk2d<ORDER, RS, LIM>, sm, true);
   if (nt < 1) return;
   fused::k_walk2d<ORDER, RS, LIM><<<(nt + nw - 1) / nw, 32 * nw, sm, f.stream>>>(f.insts, tiles, nt, parity);
 }
@@ -689,11 +696,8 @@ namespace {
 template <int ORDER, int RS, int LIM>
 void launch_vl3d(const Fused3Launch& f, int parity, const FusedTile3* tiles, int nt) {
   constexpr size_t sm = fused3::Lay<ORDER>::bytes;
-  static bool attrs = false;
-  if (!attrs) {
-    cudaFuncSetAttribute(fused3::k_vl3d<ORDER, RS, LIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    attrs = true;
-  }
+  static PerDevice attrs;
+  allow_smem(attrs, fused3::k_vl3d<ORDER, RS, LIM>, sm);
   if (nt < 1) return;
   fused3::k_vl3d<ORDER, RS, LIM><<<nt, fused3::NT, sm, f.stream>>>(f.insts, tiles, parity, f.charact_proj,
                                                                    ORDER ? f.wsmaps : nullptr);
