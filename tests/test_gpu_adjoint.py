@@ -148,6 +148,39 @@ def test_rollout_adjoint_matches_torch_autograd(nsteps, every, extra):
         assert _rel(b4.grad[v, 0], ab[v]) < 1e-9, (v, _rel(b4.grad[v, 0], ab[v]))
 
 
+def test_rollout_adjoint_of_a_walking_grid():
+    """A grid large enough to run on the strip walks records its steps from them
+    (predictor and corrector states of every cell): its gradient against torch
+    autograd."""
+    import torch
+    import torch_vl2 as T
+    from bonzo_b200._lib import WALK_VARIANT
+    from bonzo_b200.adjoint import rollout
+    gc, opts, m, P0, B0, dt = _state("vortex_pert", 512, limiter="mc")
+    G = T.Grid(gc, face_aware=True, device="cuda")
+    gen = torch.Generator(device="cpu").manual_seed(9)
+    target = (P0[0] + 0.1 * torch.randn(P0[0].shape, generator=gen, dtype=torch.float64)).cuda()
+    p, b = P0.cuda().requires_grad_(True), B0.cuda().requires_grad_(True)
+    x, y = p, b
+    for _ in range(3):
+        x, y = T.step(G, x, y, 0.5 * dt, rs="hlld", lim="mc")
+    loss_t = ((x[0] - target) ** 2).sum()
+    ap, ab = torch.autograd.grad(loss_t, (p, b))
+    eng = device_ctx(opts, path="fused", **m)
+    assert eng.variant == WALK_VARIANT
+    shp = (9, 1) + tuple(P0.shape[1:])
+    p4 = P0.reshape(shp).cuda().requires_grad_(True)
+    b4 = B0.reshape((3,) + shp[1:]).cuda().requires_grad_(True)
+    xp, xb = rollout(p4, b4, eng, 3, 0.5 * dt, checkpoint_every=2)
+    loss = ((xp[0, 0] - target) ** 2).sum()
+    loss.backward()
+    assert abs(loss.item() - loss_t.item()) <= 1e-12 * abs(loss_t.item())
+    for v in range(9):
+        assert _rel(p4.grad[v, 0], ap[v]) < 1e-9, (v, _rel(p4.grad[v, 0], ap[v]))
+    for v in range(3):
+        assert _rel(b4.grad[v, 0], ab[v]) < 1e-9, (v, _rel(b4.grad[v, 0], ab[v]))
+
+
 def _vortex_ic(gc, v, az, gam=5.0 / 3.0, beta=4 * math.pi):
     """Differentiable vortex initial state from active-cell velocities v (2, Ny, Nx)
     and the corner potential az (Ny+1, Nx+1): faces as corner differences, cell

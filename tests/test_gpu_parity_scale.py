@@ -1,10 +1,10 @@
 """Parity of the benchmarked build at the benchmark's scale.
 
 The headline batch runs the fast build (DFMA contraction and the reciprocal
-rewrites) on the persistent TMA-fed kernels (variant 8, a batch's default),
-over blast grids of every side length the uneven sweep draws (64 ... 512).
-These tests run exactly that build and kernel variant for 100 steps and hold
-it to the method's correctness bar:
+rewrites) on the strip walks (a large batch's default), smaller batches on the
+persistent TMA-fed kernels (variant 8), over blast grids of every side length
+the uneven sweep draws (64 ... 512).  These tests run that build and both kernel
+variants for 100 steps and hold them to the method's correctness bar:
 
 * every field within 1e-9 (relative to the field's maximum) of the oracle
   after 100 steps, each instance with its own CFL dt;
@@ -24,6 +24,7 @@ import numpy as np
 import pytest
 
 from bonzo_b200 import problems as P
+from bonzo_b200._lib import WALK_VARIANT
 from helpers import device_ctx, oracle_sim, rel_err, setup_case
 
 pytestmark = pytest.mark.gpu
@@ -83,13 +84,15 @@ def _check_against_oracle(b, inst, ref):
         assert b[q].check() == 0
 
 
-def test_fast_persistent_batch_every_step(sweep):
+@pytest.mark.parametrize("variant", [8, WALK_VARIANT])
+def test_fast_persistent_batch_every_step(sweep, variant):
     """Step by step (no graph): div B on the device after every step, the
     periodic instance's mass and energy, then every instance vs the oracle."""
     from bonzo_b200._lib import Batch
     inst, ref = sweep
     b = Batch([g for g, *_ in inst], **METHOD)
-    b.set_variant(8)
+    b.set_variant(variant)
+    assert b.variant == variant
     for q, (grid, gc, prim, bfld) in enumerate(inst):
         b[q].set_state(prim, bfld)
         b[q].init()
@@ -109,12 +112,14 @@ def test_fast_persistent_batch_every_step(sweep):
     _check_against_oracle(b, inst, ref)
 
 
-def test_fast_persistent_batch_graph(sweep):
+@pytest.mark.parametrize("variant", [8, WALK_VARIANT])
+def test_fast_persistent_batch_graph(sweep, variant):
     """The bench's stepping: 100 steps replayed from the captured CUDA graph."""
     from bonzo_b200._lib import Batch
     inst, ref = sweep
     b = Batch([g for g, *_ in inst], **METHOD)
-    b.set_variant(8)
+    b.set_variant(variant)
+    assert b.variant == variant
     for q, (grid, gc, prim, bfld) in enumerate(inst):
         b[q].set_state(prim, bfld)
         b[q].init()

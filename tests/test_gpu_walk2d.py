@@ -4,9 +4,12 @@ shapes of small single grids.
 Both build from the same expressions as the tile kernels, so in the exact build
 the states must be equal bit for bit: a batch that walks against the same batch
 on the tile variant 9, a single grid against the split path, which shares no
-kernel with either.  Sizes put the strips' edges everywhere: one column or row
-more and less than a strip holds, grids of a few cells, both sides of the size
-where a batch or a grid starts to walk."""
+kernel with either.  The fast build's walks round like its tiles too (they fix
+by hand what the compiler would contract another way), so there as well a batch
+that walks must equal one on tiles.  Sizes put the strips' edges everywhere: one
+column or row more and less than a strip holds, grids of a few cells, both sides
+of the size where a batch or a grid starts to walk.  (The walks against the
+oracle over 100 steps: test_gpu_parity_scale.py.)"""
 import numpy as np
 import pytest
 
@@ -124,7 +127,7 @@ def test_variant_numbers_mean_one_kernel_each():
                                (500, 500), (501, 500), (640, 397)])
 @pytest.mark.parametrize("bc", BCS[:2])
 def test_single_grid_shapes_bitwise_vs_split(n, bc):
-    """14 x 14 tiles, 16 x 16 tiles and (from 250 000 cells) walks of one grid."""
+    """14 x 14 tiles, 32 x 8 tiles and (from 250 000 cells) walks of one grid."""
     s = _state(n, bc, n[0])
     out = []
     for path in ("fused", "split"):
@@ -133,6 +136,44 @@ def test_single_grid_shapes_bitwise_vs_split(n, bc):
         c.init()
         for _ in range(2):
             c.step(0.2 / max(n) / 4)
+        out.append(c.get_state())
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("bc", BCS)
+@pytest.mark.parametrize("kw", [dict(), dict(limiter="mc"), dict(limiter="mm", grav=(0.1, -0.4, 0.2)),
+                                dict(rsolver="hll", limiter="mc"), dict(rsolver="hllt"),
+                                dict(rsolver="hllt", limiter="mm", grav=(0.1, -0.4, 0.2))],
+                         ids=lambda k: "-".join(str(v) for v in k.values()) or "default")
+def test_fast_walks_round_like_tiles(bc, kw):
+    sizes = SMALL + [(200, 151), (256, 256)]
+    grids = [dict(Nx=n[0], Ny=n[1], Nz=1, dims=2, bc=bc) for n in sizes]
+    out = []
+    for v in (WALK_VARIANT, 8, 9):
+        b = Batch(grids, cour=0.3, **kw)
+        b.set_variant(v)
+        for q, n in enumerate(sizes):
+            b[q].set_state(*_state(n, bc, q))
+            b[q].init()
+        b.advance(1e30, 5)
+        out.append([c.get_state() + (np.array(c.time()),) for c in b.instances])
+    for o in out[1:]:
+        for n, s, s0 in zip(sizes, o, out[0]):
+            assert all(np.array_equal(x, y) for x, y in zip(s, s0)), n
+
+
+@pytest.mark.parametrize("kw", [dict(grav=(0.1, -0.3, 0.0), drive_f0=0.8, drive_tau=0.05, drive_nmod=2, drive_seed=3),
+                                dict(drive_f0=0.5, drive_tau=0.1, drive_nmod=1, drive_seed=7, rsolver="hll")])
+def test_driven_walking_grid_bitwise_vs_split(kw):
+    n, bc = (520, 490), BCS[0]
+    out = []
+    for path in ("fused", "split"):
+        c = Context(Nx=n[0], Ny=n[1], Nz=1, dims=2, bc=bc, exact_fp=True, cour=0.3, path=path, **kw)
+        assert c.variant == (WALK_VARIANT if path == "fused" else -1)
+        c.set_state(*_state(n, bc, 2))
+        c.init()
+        c.advance(1e30, max_steps=3)
         out.append(c.get_state())
     for x, y in zip(*out):
         assert np.array_equal(x, y)
