@@ -37,13 +37,13 @@ BYTES_PER_ZONE = 192  # 9 conserved + 3 face-B doubles read once and written onc
 # b^(n+1) (3): 36 doubles per active zone.  The predictor reads 12 and writes
 # 12 per zone it covers (active zones plus two ghost rings).
 CORR_BYTES_PER_ZONE = 288
-# Per kernel variant, from ncu captures on the first 16 instances of this batch
-# (scaled per zone): DRAM bytes per active zone of one corrector launch
+# Per kernel variant, from ncu captures on this batch (the walks) or on its first
+# 16 instances (variant 8; scaled per zone): DRAM bytes per active zone of one corrector launch
 # (dram__bytes_read.sum + dram__bytes_write.sum), and FP64 flops per zone-update
 # of predictor and corrector (2 x DFMA + DADD + DMUL thread instructions, those
 # of the division and square-root sequences included).  Null for a variant that
 # was not captured.
-COUNTS = {8: dict(traffic=269.9, flops=1196 + 1343)}
+COUNTS = {8: dict(traffic=269.9, flops=1196 + 1343), 10: dict(traffic=298.8, flops=1017 + 1161)}
 NO_COUNTS = dict(traffic=None, flops=None)
 
 
@@ -375,7 +375,8 @@ def run_ours(args, rank, world, dist):
             "frac": round(fp64_achieved / fp64_peak, 4) if fp64_achieved and fp64_peak > 0 else None,
             "flops_per_zone": counts["flops"],
             "peak_source": "measured in this run (bnz_fp64_fma_peak: independent FMA chains on every SM)",
-            "flops_source": "ncu FP64 instruction counts of the kernels that ran, on the first 16 instances"}
+            "flops_source": "ncu FP64 instruction counts of the kernels that ran (k_walk2d: this batch; tiles: its "
+                            "first 16 instances)"}
     step_achieved = BYTES_PER_ZONE * zones / (ms_step * 1e-3) / 1e9
     step_roof = {"achieved": round(step_achieved, 1), "frac": round(step_achieved / peak, 4),
                  "bytes_per_zone": BYTES_PER_ZONE,

@@ -147,8 +147,8 @@ __global__ void k_cfl_dt(GridDev g, const double* __restrict__ w, DtState* ds, i
   dt_of_max(ds, mx, cour, clip);
 }
 
-// The same in three launches, for the instances of a split batch (whose launch
-// count reports them).
+// The same in three launches, for the instances of a split batch: the launches
+// that its captured step and bnz_batch_launch_count are tested to hold.
 __global__ void k_dt_reset(DtState* ds) { ds->cdsmax_bits = 0ULL; }
 
 __global__ void k_cds_max(GridDev g, const double* __restrict__ w, unsigned long long* slot, int hydro) {

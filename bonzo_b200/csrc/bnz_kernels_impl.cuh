@@ -291,11 +291,13 @@ namespace {
 // Planes a block of k_ee, k_update or k_update_tma walks: 16, or on a grid of
 // few columns as many as leave the launch `want` blocks, at least 2.  A block
 // walks its planes one after the other, so a small grid wants shorter walks; a
-// walk's first plane costs loads that the next ones carry.  Measured, us for 6
-// or 8 steps of one grid alone (with three in flight), 16 planes throughout
-// against this: 97 x 65 x 50 2466 (1647) against 1930 (1639), 63^3 2976 (1782)
-// against 2074 (1782), 40^3 in the TMA form 1656 (757) against 976 (600); from
-// 128^3 up it is 16.
+// walk's first plane costs loads that the next ones carry, which counts once the
+// device is full.  Measured, us a step of one grid alone (with three in flight),
+// 16 planes in all three kernels / as chosen here / 2 planes: 41^3 251 (117) / 97
+// (77) / 97 (76), 63^3 351 (208) / 242 (206) / 237 (218), 97 x 65 x 50 374 (248)
+// / 292 (250) / 297 (271), 95^3 669 (573) / 659 (574) / 626 (624); in the TMA
+// form 40^3 181 (88) / 99 (66) / 95 (72), 64^3 264 (188) / 232 (192) / 231 (202);
+// from 128^3 up it is 16.
 inline int update_kz(const plain::Box& b, int want) {
   const int cols = ((b.hi.x - b.lo.x + 32) / 32) * ((b.hi.y - b.lo.y + 8) / 8);
   for (int kz = 16; kz > 2; kz /= 2)
@@ -391,8 +393,9 @@ int split_stage(const StepArgs& a, const plain::Box& b, const double* w, double*
     const int kz = update_kz(be, 2 * sm_count());
     split::k_ee<<<cell_grid(be, kz), dim3(32, 8), 0, a.stream>>>(g, w, a.flx[0], a.flx[1], a.flx[2], a.ee, be, kz);
   }
-  // (two blocks fit an SM without TMA, one with)
-  const int kz = update_kz(b, g.dims == 3 && a.smaps ? 60 : 200);
+  // blocks wanted: where two fit an SM (k_update) more of them than where one
+  // does (k_update_tma, whose block keeps a plane's loads in flight besides)
+  const int kz = update_kz(b, g.dims == 3 && a.smaps ? 2 * sm_count() / 5 : 4 * sm_count() / 3);
   if (g.dims == 3 && a.smaps) {
     // the TMA-fed form (3D, even Ntot_x)
     constexpr size_t sm = sizeof(split::TmaSmem);

@@ -1,22 +1,28 @@
-// bnz_walk2d.cuh -- the 2D stages of a batch as strip walks of single warps.
+// bnz_walk2d.cuh -- the 2D stages as strip walks of single warps: large batches
+// and large single grids (bnz_common.h: batch_walks, grid_variant).
 //
-// A warp owns a strip of at most 30 columns and walks its rows upwards; lane l is column x0 - 1 + l, so the strip and one column on
-// either side fill the warp.  Per row it forms the y faces below the row, the
-// x faces of the row and the corner EMFs between them, then finishes the row
-// below: fluxes are used as they are formed and never stored for a tile.
+// A warp owns a strip of at most 30 columns and walks its rows upwards; lane l
+// is column x0 - 1 + l, so the strip and one column on either side fill the
+// warp.  Per row it forms the y faces below the row, the x faces of the row and
+// the corner EMFs between them, then finishes the row below: fluxes are used as
+// they are formed and never stored for a tile.
 // What a lane carries from row to row (the lower y fluxes, the row's x flux
 // differences, then its half-done update, a corner EMF, a cell EMF) stays in
 // its own slots of shared memory; values of a neighbouring column come by
 // shuffles.  The next row's cells are copied in (cp.async) while this one
 // computes.  There is no block barrier anywhere, which is what held the tile
-// kernels of bnz_fused.cuh up most (their six phases a tile end in one each),
-// and a strip forms 2.1-2.3 faces a cell where 15 x 14 tiles form 2.43.
-// Expressions are stage_cell's and the flux stages', so the bits are the same.
+// kernels of bnz_fused.cuh up most (their six phases a tile end in one each).
+// The face work is about theirs: a strip of w x h cells forms (w + 1)(h + 2) x
+// faces and (w + 2)(h + 1) y faces, 2.2 a cell at 30 x 32, 2.3 at 30 x 18 (5 M
+// zones), 2.5 at 30 x 8, against 2.43 of 15 x 14 tiles.
+// Expressions are stage_cell's and the flux stages', and what the fast build
+// would contract another way is fixed by hand, so the bits are the same in both
+// builds (test_gpu_walk2d.py).
 // What bounds it is FP64 dependency latency at 12 (corrector: 15.8 KB of shared
 // memory and 168 registers a thread) and 16 (predictor) warps an SM.  Measured,
-// HLLD, 64 blasts of 4.8 M zones, 10 steps with loading and reading the state:
-// 21.5 -> 18.1 ms against the persistent 15 x 14 tiles; one 1024^2 grid 596 ->
-// 421 us a step against 32 x 8 tiles (bnz_common.h has the sizes between).
+// HLLD, 64 blasts of 6.4 M zones 2.15 ms a step against 2.35 on the persistent
+// 15 x 14 tiles (corrector 1.27 against 1.52); one 1024^2 grid 411 us a step
+// against 596 on 32 x 8 tiles (bnz_common.h has other sizes and solvers).
 // Included inside the per-floating-point-mode namespace, after bnz_fused.cuh
 // and bnz_split_flux.cuh (cp.async helpers).
 #pragma once
