@@ -313,12 +313,19 @@ inline dim3 cell_grid(const plain::Box& b, int kz) {
 // Faces a thread of a column walk takes: as few as put all walks on the device
 // at once, up to 16 (a second wave of a few blocks costs a whole walk); a larger
 // box takes about four waves of walks of at most 32 faces (an even last wave).
+// A PLM walk starts with a slope that its neighbour forms too, so walks on 3D
+// boxes take at least 4 faces, or 2 or 1 where those would leave the device
+// emptier than half a wave: shorter ones gain up to 8 % on a grid alone (48^3
+// 128 / 134 us a step) and lose 1 to 3 % with three in flight (56^3 HLL 128 /
+// 126).  On 2D boxes, whose walks are few, a grid alone loses more by longer
+// ones (300^2 with characteristic slopes 81 / 89).
 // Measured, us a step of one grid, against four waves of at least four faces
-// with a column's walks in blocks of their own: 201 x 150 48 / 52 (HLLD, split
-// path), 30 x 3000 81 / 98, 512^2 with characteristic slopes 175 / 200, 32^3 75
-// / 83, 64^3 232 / 237; from 96^3 up the same.
-inline int walk_len(long long nf, long long ncol, long long room) {
-  for (int len = 1; len <= 16; ++len)
+// with a column's walks in blocks of their own: 201 x 150 48 / 54 (HLLD, split
+// path), 30 x 3000 81 / 98, 512^2 with characteristic slopes 168 / 200, 64^3 231
+// / 237; from 96^3 up the same.
+inline int walk_len(long long nf, long long ncol, long long room, bool d3) {
+  const long long faces = nf * ncol;
+  for (int len = !d3 || faces < room / 4 ? 1 : faces < room ? 2 : 4; len <= 16; ++len)
     if (ncol * ((nf + len - 1) / len) <= room) return len;
   const long long parts = std::max((4 * room + ncol - 1) / ncol, (nf + 31) / 32);
   return (int)((nf + parts - 1) / parts);
@@ -350,7 +357,7 @@ void launch_split_flux(const StepArgs& a, const double* w, const double* bf, con
     constexpr int sm = split::ColSmem<ORDER, CP>::BYTES;
     const int res = flux_resident(split::k_flux_march<AX, ORDER, RS, CP>, sm, per_sm);
     const long long nf = AX == 1 ? ny : nz, ncol = nx * (AX == 1 ? nz : ny);
-    const int len = walk_len(nf, ncol, (long long)res * NT), parts = (int)((nf + len - 1) / len);
+    const int len = walk_len(nf, ncol, (long long)res * NT, a.g.dims == 3), parts = (int)((nf + len - 1) / len);
     split::k_flux_march<AX, ORDER, RS, CP><<<(unsigned)((ncol * parts + NT - 1) / NT), NT, sm, a.stream>>>(
         a.g, w, bf, a.flx[AX], b, a.limiter, len, parts, a.err);
   }
